@@ -207,6 +207,7 @@ extern "C" int seismic_batch_create(const seismic_catalog *catalogs, int n_catal
     pa.twiddles = tw;
     pa.couple_begin = 0;
     pa.couple_end = pair_couples_total(c.n_events, te.tile);
+    set_pair_scales(pa);
 
     const int ng = groups_per_cta(P);
     const long long row_pairs = (rows + 1) / 2;

@@ -39,10 +39,35 @@ __device__ __forceinline__ int pad16(int i) { return i + (i >> 4); }
 template <int P> __host__ __device__ constexpr int padded_len() { return P + P / 16; }
 
 // ---------------------------------------------------------------- complex ops
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+// The inverse direction (the pair loop) runs its adds and twiddle products on
+// packed FP32 pairs: one add / mul / fma.f32x2 instruction does what two
+// scalar ones do in one issue slot (and two cycles of the FMA pipe), and
+// swapped, repeated or negated halves of an operand cost no instruction
+// (counted with ncu).  Every rounding is spelled out, so the results do not
+// depend on what the compiler contracts.  The pair loop was bound by issue and
+// latency (issue active 64 %, FMA pipe 32 %).
+template <int DIR> __device__ __forceinline__ float2 cadd(float2 a, float2 b) {
+  if constexpr (DIR > 0) return __fadd2_rn(a, b);
+  else return make_float2(a.x + b.x, a.y + b.y);
+}
+template <int DIR> __device__ __forceinline__ float2 csub(float2 a, float2 b) {
+  if constexpr (DIR > 0) return __fadd2_rn(a, make_float2(-b.x, -b.y));
+  else return make_float2(a.x - b.x, a.y - b.y);
+}
+// a b: the products with a.y are rounded, those with a.x fused.  In scalar
+// instructions: its operands are compile-time constants (immediates) or
+// the powers of a root, whose register pairs cost spills (packed powers at P =
+// 1024 with one channel, N=3000: 6.14 ms against 6.06).
+template <int DIR> __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
+  if constexpr (DIR > 0)
+    return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
+  else return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+// a b for a twiddle b: the products with b.y are rounded, those with b.x fused.
+template <int DIR> __device__ __forceinline__ float2 cmul_twiddle(float2 a, float2 b) {
+  if constexpr (DIR > 0)
+    return __ffma2_rn(a, make_float2(b.x, b.x), __fmul2_rn(make_float2(a.y, a.x), make_float2(-b.y, b.y)));
+  else return cmul<DIR>(a, b);
 }
 // a * (DIR * i)
 template <int DIR> __device__ __forceinline__ float2 mul_i(float2 a) {
@@ -70,30 +95,30 @@ template <int DIR, int K, int N> __device__ __forceinline__ float2 twc(float2 v)
     // k odd: 1, 3, 5, 7 -> (+-h, +-h)
     constexpr float c = (k == 1 || k == 7) ? h : -h;
     constexpr float s = (k == 1 || k == 3) ? h : -h;
-    return cmul(v, make_float2(c, DIR * s));
+    return cmul<DIR>(v, make_float2(c, DIR * s));
   } else {
     static_assert(N == 16, "twc: unsupported N");
     // k odd in 1..15: cos/sin of k*pi/8
     constexpr float cs[16] = {1.f, c1, h, s1, 0.f, -s1, -h, -c1, -1.f, -c1, -h, -s1, 0.f, s1, h, c1};
     constexpr float sn[16] = {0.f, s1, h, c1, 1.f, c1, h, s1, 0.f, -s1, -h, -c1, -1.f, -c1, -h, -s1};
-    return cmul(v, make_float2(cs[k], DIR * sn[k]));
+    return cmul<DIR>(v, make_float2(cs[k], DIR * sn[k]));
   }
 }
 
 // ------------------------------------------------------------ radix kernels
 template <int DIR> __device__ __forceinline__ void dft2(float2 &a, float2 &b) {
   const float2 t = a;
-  a = cadd(t, b);
-  b = csub(t, b);
+  a = cadd<DIR>(t, b);
+  b = csub<DIR>(t, b);
 }
 
 template <int DIR> __device__ __forceinline__ void dft4(float2 &v0, float2 &v1, float2 &v2, float2 &v3) {
-  const float2 s02 = cadd(v0, v2), d02 = csub(v0, v2);
-  const float2 s13 = cadd(v1, v3), d13 = mul_i<DIR>(csub(v1, v3));
-  v0 = cadd(s02, s13);
-  v2 = csub(s02, s13);
-  v1 = cadd(d02, d13);
-  v3 = csub(d02, d13);
+  const float2 s02 = cadd<DIR>(v0, v2), d02 = csub<DIR>(v0, v2);
+  const float2 s13 = cadd<DIR>(v1, v3), d13 = mul_i<DIR>(csub<DIR>(v1, v3));
+  v0 = cadd<DIR>(s02, s13);
+  v2 = csub<DIR>(s02, s13);
+  v1 = cadd<DIR>(d02, d13);
+  v3 = csub<DIR>(d02, d13);
 }
 
 // DFT_R in place on v[0..R), natural order in and out.
@@ -111,10 +136,10 @@ template <int R, int DIR> __device__ __forceinline__ void dft(float2 *v) {
     o1 = twc<DIR, 1, 8>(o1);
     o2 = twc<DIR, 2, 8>(o2);
     o3 = twc<DIR, 3, 8>(o3);
-    v[0] = cadd(e0, o0); v[4] = csub(e0, o0);
-    v[1] = cadd(e1, o1); v[5] = csub(e1, o1);
-    v[2] = cadd(e2, o2); v[6] = csub(e2, o2);
-    v[3] = cadd(e3, o3); v[7] = csub(e3, o3);
+    v[0] = cadd<DIR>(e0, o0); v[4] = csub<DIR>(e0, o0);
+    v[1] = cadd<DIR>(e1, o1); v[5] = csub<DIR>(e1, o1);
+    v[2] = cadd<DIR>(e2, o2); v[6] = csub<DIR>(e2, o2);
+    v[3] = cadd<DIR>(e3, o3); v[7] = csub<DIR>(e3, o3);
   } else {
     static_assert(R == 16, "dft: unsupported radix");
     // r = r1 + 4 r2 ; DFT4 over r2 for each r1 ; twiddle w16^{r1 q2} ; DFT4 over r1 ; X[q2 + 4 q1]
@@ -146,19 +171,19 @@ template <int DIR> __device__ __forceinline__ float2 twiddle_lookup(const float2
 
 // v[r] *= w^r, r = 1..R-1, w = exp(DIR 2 pi i m / (NS R)); powers from one
 // table entry and a shallow product tree (at most 4 roundings per power).
-template <int R> __device__ __forceinline__ void root_powers(float2 w1, float2 (&w)[R]) {
+template <int R, int DIR> __device__ __forceinline__ void root_powers(float2 w1, float2 (&w)[R]) {
   w[1] = w1;
 #pragma unroll
-  for (int r = 2; r < R; ++r) w[r] = (r & 1) ? cmul(w[r - 1], w1) : cmul(w[r / 2], w[r / 2]);
+  for (int r = 2; r < R; ++r) w[r] = (r & 1) ? cmul<DIR>(w[r - 1], w1) : cmul<DIR>(w[r / 2], w[r / 2]);
 }
-template <int R> __device__ __forceinline__ void apply_powers(float2 *v, const float2 (&w)[R]) {
+template <int R, int DIR> __device__ __forceinline__ void apply_powers(float2 *v, const float2 (&w)[R]) {
 #pragma unroll
-  for (int r = 1; r < R; ++r) v[r] = cmul(v[r], w[r]);
+  for (int r = 1; r < R; ++r) v[r] = cmul_twiddle<DIR>(v[r], w[r]);
 }
-template <int R> __device__ __forceinline__ void apply_root_powers(float2 *v, float2 w1) {
+template <int R, int DIR> __device__ __forceinline__ void apply_root_powers(float2 *v, float2 w1) {
   float2 w[R];
-  root_powers<R>(w1, w);
-  apply_powers<R>(v, w);
+  root_powers<R, DIR>(w1, w);
+  apply_powers<R, DIR>(v, w);
 }
 
 template <int P, int R, int NS, int DIR>
@@ -167,7 +192,7 @@ __device__ __forceinline__ void apply_twiddles(float2 *v, int m, const float2 *_
     return;
   } else {
     constexpr int step = kMaxP / (NS * R);
-    apply_root_powers<R>(v, twiddle_lookup<DIR>(tw, m * step));
+    apply_root_powers<R, DIR>(v, twiddle_lookup<DIR>(tw, m * step));
   }
 }
 
@@ -200,7 +225,7 @@ template <int NUM, int DEN, int DIR> __device__ __forceinline__ float2 mul_turn(
     constexpr double x = 6.28318530717958647692528676655900577 * k / DEN - 3.14159265358979323846264338327950288;
     constexpr float c = (float)(-ct_cos(x));
     constexpr float s = (float)(-ct_sin(x) * DIR);
-    return cmul(v, make_float2(c, s));
+    return cmul<DIR>(v, make_float2(c, s));
   }
 }
 
@@ -236,7 +261,7 @@ __device__ __forceinline__ void base_root_jobs(float2 (&v)[32], float2 root) {
   constexpr int G = P / 32;
   constexpr int J = 32 / R;
   if constexpr (Q < J) {
-    apply_root_powers<R>(&v[Q * R], mul_turn<Q * G, NS * R, DIR>(root));
+    apply_root_powers<R, DIR>(&v[Q * R], mul_turn<Q * G, NS * R, DIR>(root));
     dft<R, DIR>(&v[Q * R]);
     base_root_jobs<P, R, NS, DIR, Q + 1>(v, root);
   }
@@ -248,14 +273,16 @@ __device__ __forceinline__ void pass_compute_held(float2 (&v)[32], float2 root) 
   constexpr int G = P / 32;
   constexpr int J = 32 / R;
   static_assert(NS > 1 && (G % NS == 0 || J * G <= NS), "pass_compute_held: root not of one kind");
+  // the powers depend on the thread alone; without this the compiler forms them
+  // all before the item loop and spills them (up to 312 bytes a thread)
+  asm volatile("" : "+f"(root.x), "+f"(root.y));
   if constexpr (G % NS == 0) {
     float2 w[R];
-    root_powers<R>(root, w);
+    root_powers<R, DIR>(root, w);
 #pragma unroll
-    for (int q = 0; q < J; ++q) {
-      apply_powers<R>(&v[q * R], w);
-      dft<R, DIR>(&v[q * R]);
-    }
+    for (int q = 0; q < J; ++q) apply_powers<R, DIR>(&v[q * R], w);
+#pragma unroll
+    for (int q = 0; q < J; ++q) dft<R, DIR>(&v[q * R]);
   } else {
     base_root_jobs<P, R, NS, DIR>(v, root);
   }
@@ -327,10 +354,10 @@ __device__ __forceinline__ void pass_compute(float2 (&v)[32], int t, const float
   if constexpr (NS > 1 && J > 1 && G % NS == 0) {
     // every job of this thread has the same m = t mod NS: one set of powers
     float2 w[R];
-    root_powers<R>(roots != nullptr ? roots[0] : twiddle_lookup<DIR>(tw, (t % NS) * (kMaxP / (NS * R))), w);
+    root_powers<R, DIR>(roots != nullptr ? roots[0] : twiddle_lookup<DIR>(tw, (t % NS) * (kMaxP / (NS * R))), w);
 #pragma unroll
     for (int q = 0; q < J; ++q) {
-      apply_powers<R>(&v[q * R], w);
+      apply_powers<R, DIR>(&v[q * R], w);
       dft<R, DIR>(&v[q * R]);
     }
   } else {
@@ -338,7 +365,7 @@ __device__ __forceinline__ void pass_compute(float2 (&v)[32], int t, const float
     for (int q = 0; q < J; ++q) {
       const int j = t + q * G;
       if (roots != nullptr)
-        apply_root_powers<R>(&v[q * R], roots[q]);
+        apply_root_powers<R, DIR>(&v[q * R], roots[q]);
       else
         apply_twiddles<P, R, NS, DIR>(&v[q * R], j % NS, tw);
       dft<R, DIR>(&v[q * R]);

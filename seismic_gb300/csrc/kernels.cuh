@@ -1,6 +1,7 @@
 // Kernel declarations and launch helpers shared by the C-ABI layer.
 #pragma once
 
+#include <cmath>
 #include <cstddef>
 #include <cstdint>
 #include <cstdlib>
@@ -106,6 +107,10 @@ struct PairArgs {
   float threshold;
   int n_hist;              // 0 disables histograms
   float delta_hist;        // float(1.0 / n_hist)
+  // set by the launch (set_pair_scales): 1 / delta_hist rounded, and 1 /
+  // n_channels as hi + lo floats, the scale of prescaled spectra
+  float inv_delta_hist;
+  float2 channel_scale;
   float *vals_pos;
   int *lags_pos;
   float *vals_neg;
@@ -161,6 +166,14 @@ struct PairArgs {
   // -- the deterministic way for a test to take the abort path.
   int wait_probe;
 };
+
+// Fills the PairArgs constants that every epilogue would otherwise divide for.
+inline void set_pair_scales(PairArgs &a) {
+  a.inv_delta_hist = a.delta_hist > 0.f ? 1.0f / a.delta_hist : 0.f;
+  const float c = (float)a.n_channels;
+  const float h = 1.0f / c;
+  a.channel_scale = make_float2(h, std::fma(-h, c, 1.0f) / c);  // 1 - h c exact by FMA
+}
 
 // SEISMIC_DEVICE_WAIT_PROBE set to a nonzero value.
 inline int device_wait_probe() {

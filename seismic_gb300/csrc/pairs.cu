@@ -157,7 +157,7 @@ __device__ __forceinline__ void pair_body(const PairArgs &a, long long w_first, 
     float2 v[32];
     assemble_couple(y, t, v);
     inverse_fft_group<P>(v, buf, t, g, ca, cb, a.twiddles, roots);
-    scan_and_write<P, kLivenessVote<P, ST>, kScanRowSkip<P, ST>>(a, v, i, ja, i, jb, out_b, t, g, red, hist, smem_hist, wmask, buf);
+    scan_and_write<P, kLivenessVote<P, ST>>(a, v, i, ja, i, jb, out_b, t, g, red, hist, smem_hist, wmask, buf);
   }
 }
 
@@ -342,7 +342,9 @@ template <int P> static size_t pair_smem_bytes(int n_hist) {
   return s;
 }
 
-template <int P, int ST> static cudaError_t launch_pairs_st(const PairArgs &a, int grid, cudaStream_t s) {
+template <int P, int ST> static cudaError_t launch_pairs_st(const PairArgs &a0, int grid, cudaStream_t s) {
+  PairArgs a = a0;
+  set_pair_scales(a);
   constexpr int G = P / 32;
   constexpr int NG = (256 / G) > 0 ? (256 / G) : 1;
   const size_t smem = pair_smem_bytes<P>(a.n_hist);

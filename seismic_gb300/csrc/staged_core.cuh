@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(NWARP * 32 + 32, 1)
         else
           inverse_fft_group<P>(v, buf, t, g, ca, cb, a.twiddles, roots, &stop);
         if (stop) break;
-        scan_and_write<P, kLivenessVote<P, ST>, kScanRowSkip<P, ST>>(a, v, i, ja, i, jb, out_b, t, g, red, hist, smem_hist, wmask, buf);
+        scan_and_write<P, kLivenessVote<P, ST>>(a, v, i, ja, i, jb, out_b, t, g, red, hist, smem_hist, wmask, buf);
       } else if (group_sync_any<G>(g, stop)) {
         break;
       }
@@ -479,6 +479,7 @@ static cudaError_t launch_staged_t(const PairArgs &a0, int sm_count, cudaStream_
   using SH = Staged<P, NWARP, RU, ST>;
   using ST_T = typename SpecT<ST>::T;
   PairArgs a = a0;
+  set_pair_scales(a);
   a.item_i = staged_item_rows(SH::NG, a);
   if (KTI && a.item_i != KTI) return cudaErrorInvalidConfiguration;  // the caller picks KTI from this rule
   const StagedGeom gm = staged_geom(SH::NG, a.item_i);
