@@ -23,7 +23,7 @@
 // a ring of K shared-memory slots: two 3-D TMA boxes {S bins, 1 channel, TI
 // or TJ events} (rows past the last event are zero-filled by the TMA unit),
 // completing on the slot's `full` mbarrier; the FFT warps conj-multiply
-// from the slot and release it on its `empty` mbarrier.  While the groups
+// from the slot and release it on its `empty` mbarrier, one arrive a warp.  While the groups
 // run their inverse FFTs the producer fills the ring with the next item's
 // units, so spectra reads leave the critical path.  A unit stages TI + TJ
 // rows for TI TJ pairs, each row shared by all the groups that use it: with
@@ -67,19 +67,28 @@ template <int P, int NWARP, int RU, int ST> struct Staged {  // RU: chunks r per
   static constexpr int G = P / 32;
   static constexpr int NG = NWARP * 32 / G;  // FFT groups per CTA
   static constexpr int S = P / 16;
+  // Chunks per TMA box: as many of a slot's as a box row (256 elements) takes,
+  // so a unit is two copies of long rows instead of two per chunk.  Q=512 x 4,
+  // N=6000: 18.0 -> 17.7 ms; P=1024 with three channels, N=2500: 5.69 -> 5.57.
+  static constexpr int BX = RU * S <= 256 ? RU : (256 / S < RU ? 256 / S : RU);
   static constexpr int NW = (G + 31) / 32;
   static constexpr int CONSUMERS = NWARP * 32;  // FFT threads
   static constexpr int THREADS = CONSUMERS + 32;  // + the producer warp
-  // exchange buffer of one group.  P = 4096 with FP32 spectra runs its
-  // exchanges in two halves (inverse_fft_group_split) and leaves the other
-  // half to the ring: N=4096 C=3 94.6 -> 102.3 M pairs/s.  Elsewhere the
-  // extra barriers cost more than the ring gains (measured, M pairs/s,
-  // full / split exchange): FP16 spectra at that shape 102.5 / 92.0; the
-  // overlap-save Q=512 x 4 form 831 / 813; Q=1024 x 2 with three channels
-  // 340 / 336; plain P=2048 one channel 268 / 262 -- only plain P=2048 with
-  // three channels gained (198 / 211).
-  static constexpr bool SPLIT_EX = P == 4096 && ST == 0;
+  // Exchange buffer of one group.  FP32 spectra: half a transform
+  // (inverse_fft_group_split runs each exchange in two rounds); the other half
+  // goes to the ring, which then holds an item or most of one, where the FFT
+  // threads waited for an item's last units while the ring refilled one copy
+  // latency at a time.  Measured with one arrive a warp and long box rows, ms
+  // before / after: Q=1024 x 2 frames of three channels (N=3000) 12.4 / 10.4, plain P=2048
+  // with three channels (N=2000) 8.86 / 7.39, P=2048 (N=3000) 13.6 / 12.6, Q=512 x 4
+  // (N=6000) 18.5 / 17.6, P=1024 with three channels (N=2500) 5.69 / 5.46.  Half types' items
+  // are half as long and gain nothing from a deeper ring (FP16 Q=512 x 4 17.28 / 17.39).
+  static constexpr bool SPLIT_EX = ST == 0;
   static constexpr int EX_LEN = SPLIT_EX ? padded_len<P / 2>() : padded_len<P>();
+  // A unit's barrier is polled while the one before it is multiplied: hides the
+  // poll behind the half types' longer products (FP16 Q=1024 x 2, three channels, N=1733
+  // 3.37 / 3.16 ms), costs FP32 1-3 % (Q=512 x 4 17.6 / 17.9).
+  static constexpr bool EARLY_POLL = ST != 0;
   static constexpr size_t EX_BYTES = (size_t)NG * EX_LEN * sizeof(float2);
   static constexpr size_t RED_BYTES = (size_t)NG * NW * 8 * sizeof(unsigned);
   static constexpr size_t PROD_OFF = (EX_BYTES + RED_BYTES + 15) / 16 * 16;
@@ -156,6 +165,12 @@ __device__ __forceinline__ bool consumer_wait(uint64_t *bar, uint32_t parity, vo
   }
 }
 
+// The same, answered alike on all 32 lanes of the calling warp (a lane that
+// polls later may see a copy land that another gave up on): the warp reads a
+// unit, or leaves, as one.
+__device__ __forceinline__ bool consumer_wait_warp(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
+  return __all_sync(0xffffffffu, consumer_wait(bar, parity, abort_flag));
+}
 
 // Default poll limit of the producer's waits (with back-off: seconds).
 constexpr uint32_t kStagedWaitPolls = 1u << 24;
@@ -182,10 +197,10 @@ __device__ __forceinline__ void staged_issue(const PairArgs &a, const StagedGeom
   const int c = cur->c, r = cur->r;
   tc::mbar_arrive_expect_tx(full, RU * sub_bytes);
 #pragma unroll
-  for (int h = 0; h < RU; ++h) {
+  for (int h = 0; h < RU; h += SH::BX) {
     unsigned char *d = dst + h * sub_bytes;
     tc::tma_load_3d(d, imap, (r + h) * S, c, (int)cur->i, full);
-    tc::tma_load_3d(d + ibytes, jmap, (r + h) * S, c, (int)cur->j0, full);
+    tc::tma_load_3d(d + SH::BX * ibytes, jmap, (r + h) * S, c, (int)cur->j0, full);
   }
   cur->r += RU;
   if (cur->r == 8) {
@@ -242,7 +257,7 @@ __global__ void __launch_bounds__(NWARP * 32 + 32, 1)
     tc::mbar_init(probe, 1);
     for (int k = 0; k < K; ++k) {
       tc::mbar_init(&full[k], 1);
-      tc::mbar_init(&empty[k], SH::CONSUMERS);
+      tc::mbar_init(&empty[k], NWARP);  // one arrive a warp
     }
     tc::fence_mbarrier_init();
     tc::fence_proxy_async_smem();
@@ -308,12 +323,13 @@ __global__ void __launch_bounds__(NWARP * 32 + 32, 1)
       // the item's first unit being full also publishes its (i, j0); if it
       // never landed, the entry read below is stale, and nothing indexes
       // memory with it before the group's vote after the unit loop
-      bool stop = !consumer_wait(&full[slot], phase, s_abort);
+      bool stop = !consumer_wait_warp(&full[slot], phase, s_abort);
       const StagedItem it = items[seq % kItemRing];
       // the group's i row gi and couple column gc within the item
       const int ti = KTI ? KTI : a.item_i, tjh = KTI ? KTJ / 2 : (a.item_j >> 1);
       const int gi = KTI ? g / (KTJ / 2) : (int)(((unsigned)g * a.item_magic) >> 16), gc = g - gi * tjh;
-      const int ri = gi * S, rows = KTI ? KTI + KTJ : a.item_i + a.item_j;
+      constexpr int BS = SH::BX * S;  // bins of a row in one box
+      const int ri = gi * BS, rows = KTI ? KTI + KTJ : a.item_i + a.item_j;
       const long long i = it.i + gi, j0 = it.j0;
       long long ja = j0 + 2 * gc, jb = ja + 1;
       bool live, out_b;
@@ -329,28 +345,37 @@ __global__ void __launch_bounds__(NWARP * 32 + 32, 1)
         out_b = jb - a.col_begin < a.n_cols;
         if (!out_b) jb = ja;
       }
-      const int ra = (ti + (int)(ja - j0)) * S, rb = (ti + (int)(jb - j0)) * S;  // rows of ja, jb in a chunk
+      const int ra = (ti + (int)(ja - j0)) * BS, rb = (ti + (int)(jb - j0)) * BS;  // rows of ja, jb in a chunk
       CoupleAcc y;
       y.zero();
+      // units of the item; a warp releases a slot with one arrive
+      bool ready = true;  // the first unit's wait is above
       for (int c = 0; c < C && !stop; ++c) {
 #pragma unroll
         for (int rp = 0; rp < 8; rp += RU) {
-          if (!consumer_wait(&full[slot], phase, s_abort)) {
+          if (!__all_sync(0xffffffffu, ready) && !consumer_wait_warp(&full[slot], phase, s_abort)) {
             stop = true;
             break;
           }
           const ST_T *u = reinterpret_cast<const ST_T *>(ring + (size_t)slot * UNIT);
-#pragma unroll
-          for (int h = 0; h < RU; ++h) {
-            const ST_T *uh = u + h * (rows * S);
-            if (live)
-              y.add<ST>(rp + h, uh[ri + ca], uh[ra + ca], uh[rb + ca], uh[ri + cb], uh[ra + cb], uh[rb + cb]);
-          }
-          tc::mbar_arrive(&empty[slot]);
+          uint64_t *release = &empty[slot];
           if (++slot == K) {
             slot = 0;
             phase ^= 1u;
           }
+          if constexpr (SH::EARLY_POLL) {
+            if (rp + RU < 8 || c + 1 < C) ready = tc::mbar_test_wait(&full[slot], phase);
+          } else {
+            ready = false;
+          }
+#pragma unroll
+          for (int h = 0; h < RU; ++h) {
+            const ST_T *uh = u + (h / SH::BX) * (rows * BS) + (h % SH::BX) * S;
+            if (live)
+              y.add<ST>(rp + h, uh[ri + ca], uh[ra + ca], uh[rb + ca], uh[ri + cb], uh[ra + cb], uh[rb + cb]);
+          }
+          __syncwarp();
+          if ((threadIdx.x & 31) == 0) tc::mbar_arrive(release);
         }
       }
       // an abort inside the item: the group leaves together, by the vote
@@ -514,7 +539,7 @@ static cudaError_t launch_staged_t(const PairArgs &a0, int sm_count, cudaStream_
   for (int side = 0; side < 2; ++side) {
     const cuuint64_t dims[3] = {(cuuint64_t)(P / 2), (cuuint64_t)spectrum_rows(a),
                                 (cuuint64_t)(side == 0 ? a.n_events : n_i)};
-    const cuuint32_t box[3] = {(cuuint32_t)SH::S, 1u, (cuuint32_t)(side == 0 ? gm.tj : gm.ti)};
+    const cuuint32_t box[3] = {(cuuint32_t)(SH::BX * SH::S), 1u, (cuuint32_t)(side == 0 ? gm.tj : gm.ti)};
     if (tensor_map_encoder()(side == 0 ? &map : &imap, dt, 3, const_cast<void *>(side == 0 ? a.spectra : spec_i),
                              dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
