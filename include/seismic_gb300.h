@@ -370,13 +370,25 @@ int seismic_server_destroy(seismic_server *server);
  * thresholds with the same strict comparisons).  Writes at most `capacity`
  * entries per side and the full counts to d_counts[0] (positive side) and
  * d_counts[1] (negative side); capacity 0 only counts.  `workspace` holds
- * seismic_compact_workspace_bytes(n_pairs) bytes.  Stream-ordered. */
+ * seismic_compact_workspace_bytes(n_pairs) bytes (the block counts, and one bit
+ * a pair and side that spares the write pass a second read of the values; a
+ * workspace of 16 (ceil(n_pairs / 4096) + 1) bytes, the counts alone, is taken
+ * too).  Stream-ordered. */
 size_t seismic_compact_workspace_bytes(long long n_pairs);
 int seismic_compact_pairs_device(const float *d_vals_pos, const int *d_lags_pos, const float *d_vals_neg,
                                  const int *d_lags_neg, long long n_pairs, float threshold, long long capacity,
                                  long long *d_index_pos, float *d_value_pos, int *d_lag_pos,
                                  long long *d_index_neg, float *d_value_neg, int *d_lag_neg,
                                  long long *d_counts, void *workspace, size_t workspace_bytes, void *stream);
+
+/* The write half of a compaction: the kept pairs from a `workspace` that
+ * seismic_compact_pairs_device (capacity 0, say) has filled for the same
+ * arrays, n_pairs, threshold and workspace_bytes, earlier on this stream. */
+int seismic_compact_write_device(const float *d_vals_pos, const int *d_lags_pos, const float *d_vals_neg,
+                                 const int *d_lags_neg, long long n_pairs, float threshold, long long capacity,
+                                 long long *d_index_pos, float *d_value_pos, int *d_lag_pos,
+                                 long long *d_index_neg, float *d_value_neg, int *d_lag_neg,
+                                 const void *workspace, size_t workspace_bytes, void *stream);
 
 /* Histograms of stored coefficients, accumulated into d_max_hist / d_min_hist
  * with the rule of Correlation_in_OMP/correlation_c.cpp:116-117, :128-129

@@ -13,11 +13,11 @@
 // reference's CSR matrices hold after a run with that threshold -- so only
 // those cross PCIe.
 //
-// Compaction is two passes over blocks of kCompactBlock pairs: count per
-// block, one exclusive scan of the block counts, then a write pass that ranks
-// each kept pair inside its block with warp ballots.  Output order is the
-// packed order; every pass is HBM-bound (algorithmic bytes: 8 B per pair read
-// twice for the values, plus the kept pairs' lags and outputs).
+// Compaction.  A count pass reads the values once (HBM-bound), keeps one bit a
+// pair and side (kept or not) and counts per CTA; the write pass, whose CTAs
+// own the same pairs, sums the counts before its own, reads the bits, 1/32 of
+// the values' bytes, and touches only the kept pairs.  Output order is the
+// packed order.
 #include <cstdint>
 
 #include "../../include/seismic_gb300.h"
@@ -30,163 +30,226 @@ int report_cuda(cudaError_t e, const char *what);
 void note_launches(unsigned n);
 
 constexpr int kCompactThreads = 256;
-constexpr int kCompactPerThread = 16;
-constexpr int kCompactBlock = kCompactThreads * kCompactPerThread;  // pairs per block
+constexpr int kCompactWarps = kCompactThreads / 32;
+constexpr int kCompactWords = 16;                                     // 32-pair words a warp and side
+constexpr int kCompactBlock = kCompactWarps * kCompactWords * 32;     // pairs per block
+constexpr int kHistThreads = 256;
 constexpr int kHistSmemMax = 4096;
+constexpr int kHistSmemBytes = 48 * 1024;
 
-__device__ __forceinline__ int sparse_hist_bin(float v, float delta, int n_hist) {
+// Bin of a stored coefficient, the pair kernel's rule: (int)(v / delta) with
+// the quotient rounded to nearest, by a correctly rounded reciprocal and one
+// residual step (Markstein's theorem; hist_bin in pair_core.cuh).
+__device__ __forceinline__ int sparse_hist_bin(float v, float delta, float inv, int n_hist) {
   if (v >= 1.0f) return n_hist - 1;
-  int b = (int)(v / delta);
+  const float q = v * inv;
+  const int b = (int)fmaf(fmaf(-q, delta, v), inv, q);
   return b > n_hist - 1 ? n_hist - 1 : (b < 0 ? 0 : b);
 }
 
+// The blocks that this CTA owns, a contiguous run; warp w takes chunk (512
+// pairs) w of each, so a CTA reads 16 KB runs (a run of chunks per warp read 134
+// M pairs 20 % slower).
+struct CompactRange {
+  long long b0, b1;
+};
+__device__ __forceinline__ CompactRange compact_range(long long nb) {
+  return CompactRange{(long long)blockIdx.x * nb / gridDim.x, (long long)(blockIdx.x + 1) * nb / gridDim.x};
+}
+
+// Word of this lane in chunk q: the kept bits of 32 consecutive pairs, the
+// chunk's positive word `lane` for lane < 16, its negative word lane - 16 for
+// the others.
+__device__ __forceinline__ unsigned compact_word(const float *__restrict__ vp, const float *__restrict__ vn,
+                                                 long long n, float thr, long long q, int lane) {
+  const long long e0 = q * kCompactWords * 32 + lane;
+  float p[kCompactWords], m[kCompactWords];
+#pragma unroll
+  for (int k = 0; k < kCompactWords; ++k) {  // 32 loads in flight a thread
+    const long long e = e0 + 32 * k;
+    p[k] = e < n ? __ldcs(vp + e) : 0.f;
+    m[k] = e < n ? __ldcs(vn + e) : 0.f;
+  }
+  unsigned word = 0;
+#pragma unroll
+  for (int k = 0; k < kCompactWords; ++k) {
+    const bool in = e0 + 32 * k < n;
+    const unsigned bp = __ballot_sync(0xffffffffu, in && p[k] > thr);
+    const unsigned bn = __ballot_sync(0xffffffffu, in && m[k] < -thr);
+    if (lane == k) word = bp;
+    if (lane == k + kCompactWords) word = bn;
+  }
+  return word;
+}
+
+// What bounds it: the read of both value arrays (134 M pairs: 168 us, 6.4 TB/s).
+// counts: [2][grid] kept pairs per CTA; totals: zeroed by the caller.
 __global__ void __launch_bounds__(kCompactThreads) compact_count_kernel(const float *__restrict__ vp,
                                                                           const float *__restrict__ vn,
                                                                           long long n, float thr, long long nb,
-                                                                          long long *__restrict__ counts) {
-  for (long long b = blockIdx.x; b < nb; b += gridDim.x) {
-    int cp = 0, cn = 0;
-#pragma unroll 4
-    for (int k = 0; k < kCompactPerThread; ++k) {
-      const long long e = b * kCompactBlock + k * kCompactThreads + threadIdx.x;
-      if (e < n) {
-        cp += __ldg(vp + e) > thr;
-        cn += __ldg(vn + e) < -thr;
-      }
-    }
-    const int sp = __reduce_add_sync(0xffffffffu, (unsigned)cp);
-    const int sn = __reduce_add_sync(0xffffffffu, (unsigned)cn);
-    __shared__ int s_p[kCompactThreads / 32], s_n[kCompactThreads / 32];
-    if ((threadIdx.x & 31) == 0) {
-      s_p[threadIdx.x >> 5] = sp;
-      s_n[threadIdx.x >> 5] = sn;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      long long tp = 0, tn = 0;
-      for (int w = 0; w < kCompactThreads / 32; ++w) {
-        tp += s_p[w];
-        tn += s_n[w];
-      }
-      counts[b] = tp;
-      counts[nb + b] = tn;
-    }
-    __syncthreads();
+                                                                          long long *__restrict__ counts,
+                                                                          unsigned *__restrict__ words,
+                                                                          unsigned long long *__restrict__ totals) {
+  __shared__ unsigned long long s_cnt[2];
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0;
+  __syncthreads();
+  const CompactRange r = compact_range(nb);
+  long long mine = 0;
+  for (long long b = r.b0; b < r.b1; ++b) {
+    const long long q = b * kCompactWarps + (threadIdx.x >> 5);
+    const unsigned word = compact_word(vp, vn, n, thr, q, lane);
+    if (words) words[q * 32 + lane] = word;
+    mine += __popc(word);
+  }
+  if (mine) atomicAdd(&s_cnt[lane / kCompactWords], (unsigned long long)mine);
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    counts[(long long)threadIdx.x * gridDim.x + blockIdx.x] = (long long)s_cnt[threadIdx.x];
+    if (s_cnt[threadIdx.x]) atomicAdd(&totals[threadIdx.x], s_cnt[threadIdx.x]);
   }
 }
 
-// Exclusive scan of the 2 nb block counts in place (one CTA); totals to out[0..1].
-__global__ void __launch_bounds__(1024) compact_scan_kernel(long long *__restrict__ counts, long long nb,
-                                                            long long *__restrict__ totals) {
-  __shared__ long long s[1024];
-  for (int side = 0; side < 2; ++side) {
-    long long *c = counts + side * nb;
-    const long long per = (nb + blockDim.x - 1) / blockDim.x;
-    const long long b0 = threadIdx.x * per, b1 = b0 + per < nb ? b0 + per : nb;
-    long long local = 0;
-    for (long long b = b0; b < b1; ++b) local += c[b];
-    s[threadIdx.x] = local;
-    __syncthreads();
-    for (int off = 1; off < (int)blockDim.x; off <<= 1) {  // inclusive Hillis-Steele scan
-      const long long add = threadIdx.x >= (unsigned)off ? s[threadIdx.x - off] : 0;
-      __syncthreads();
-      s[threadIdx.x] += add;
-      __syncthreads();
-    }
-    long long run = s[threadIdx.x] - local;  // exclusive prefix of this thread's segment
-    for (long long b = b0; b < b1; ++b) {
-      const long long v = c[b];
-      c[b] = run;
-      run += v;
-    }
-    if (threadIdx.x == blockDim.x - 1) totals[side] = s[threadIdx.x];
-    __syncthreads();
-  }
-}
-
+// The kept pairs of each chunk, one a lane: lane s takes the chunk's s-th kept
+// pair (a search over the words' running counts, then the bit of its rank), so
+// up to 32 gathers are in flight a warp and the stores are contiguous however
+// many are kept.  134 M pairs, 2 % kept: 238 us against 1514 with two
+// barriers per 256 pairs and 428 with a word at a time.  Without stored words
+// (a workspace that has no room for them) the values are read again.
 __global__ void __launch_bounds__(kCompactThreads) compact_write_kernel(
     const float *__restrict__ vp, const int *__restrict__ lp, const float *__restrict__ vn,
-    const int *__restrict__ ln, long long n, float thr, long long nb, const long long *__restrict__ offsets,
-    long long capacity, long long *__restrict__ idx_p, float *__restrict__ val_p, int *__restrict__ lag_p,
-    long long *__restrict__ idx_n, float *__restrict__ val_n, int *__restrict__ lag_n) {
-  __shared__ int s_p[kCompactThreads / 32], s_n[kCompactThreads / 32];
+    const int *__restrict__ ln, long long n, float thr, long long nb, const long long *__restrict__ counts,
+    const unsigned *__restrict__ words, long long capacity, long long *__restrict__ idx_p,
+    float *__restrict__ val_p, int *__restrict__ lag_p, long long *__restrict__ idx_n, float *__restrict__ val_n,
+    int *__restrict__ lag_n) {
+  __shared__ unsigned long long s_before[2];      // kept pairs of the CTAs before this one
+  __shared__ int s_warp[2][2][kCompactWarps];     // [block parity][side]: of each warp's chunk
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned below = (1u << lane) - 1u;
-  for (long long b = blockIdx.x; b < nb; b += gridDim.x) {
-    long long op = offsets[b], on = offsets[nb + b];
-    for (int k = 0; k < kCompactPerThread; ++k) {
-      const long long e = b * kCompactBlock + k * kCompactThreads + threadIdx.x;
-      float a = 0.f, c = 0.f;
-      if (e < n) {
-        a = __ldg(vp + e);
-        c = __ldg(vn + e);
-      }
-      const bool kp = e < n && a > thr, kn = e < n && c < -thr;
-      const unsigned bp = __ballot_sync(0xffffffffu, kp), bn = __ballot_sync(0xffffffffu, kn);
-      if (lane == 0) {
-        s_p[warp] = __popc(bp);
-        s_n[warp] = __popc(bn);
-      }
-      __syncthreads();
-      int wp = 0, wn = 0, tp = 0, tn = 0;
+  if (threadIdx.x < 2) s_before[threadIdx.x] = 0;
+  __syncthreads();
+  for (int sd = 0; sd < 2; ++sd) {
+    unsigned long long t = 0;
+    for (int c = threadIdx.x; c < (int)blockIdx.x; c += kCompactThreads)
+      t += (unsigned long long)counts[(long long)sd * gridDim.x + c];
+    if (t) atomicAdd(&s_before[sd], t);
+  }
+  __syncthreads();
+  long long off_p = (long long)s_before[0], off_n = (long long)s_before[1];
+  const CompactRange r = compact_range(nb);
+  for (long long b = r.b0; b < r.b1; ++b) {
+    const long long q = b * kCompactWarps + warp;
+    const unsigned word = words ? __ldg(words + q * 32 + lane) : compact_word(vp, vn, n, thr, q, lane);
+    const int c = __popc(word);
+    int incl = c;  // running count over the 16 positive words, then the 16 negative ones
 #pragma unroll
-      for (int w = 0; w < kCompactThreads / 32; ++w) {
-        if (w < warp) {
-          wp += s_p[w];
-          wn += s_n[w];
-        }
-        tp += s_p[w];
-        tn += s_n[w];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += x;
+    }
+    const int pos = __shfl_sync(0xffffffffu, incl, kCompactWords - 1), all = __shfl_sync(0xffffffffu, incl, 31);
+    int(&cnt)[2][kCompactWarps] = s_warp[b & 1];  // two sets: the next block's is written while this one is read
+    if (lane == 0) {
+      cnt[0][warp] = pos;
+      cnt[1][warp] = all - pos;
+    }
+    __syncthreads();
+    long long at_p = off_p, at_n = off_n;  // this chunk's first positive and negative pair
+    for (int w = 0; w < kCompactWarps; ++w) {
+      off_p += cnt[0][w];
+      off_n += cnt[1][w];
+      if (w < warp) {
+        at_p += cnt[0][w];
+        at_n += cnt[1][w];
       }
-      if (kp) {
-        const long long o = op + wp + __popc(bp & below);
+    }
+    for (int s0 = 0; s0 < all; s0 += 32) {
+      const int s = s0 + lane;
+      int k = 0;  // the word of the s-th kept pair: words whose running count is <= s
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const int x = __shfl_sync(0xffffffffu, incl, k + o - 1);
+        if (x <= s) k += o;
+      }
+      k = k < 31 ? k : 31;
+      const unsigned bits = __shfl_sync(0xffffffffu, word, k);
+      int rank = s - (__shfl_sync(0xffffffffu, incl, k) - __popc(bits));
+      if (s < all) {
+        int bit = 0;  // the set bit of that rank
+#pragma unroll
+        for (int w = 16; w > 0; w >>= 1) {
+          const int x = __popc((bits >> bit) & ((1u << w) - 1u));
+          if (rank >= x) {
+            rank -= x;
+            bit += w;
+          }
+        }
+        const long long e = (q * kCompactWords + (k & (kCompactWords - 1))) * 32 + bit;
+        const bool neg = s >= pos;
+        const long long o = neg ? at_n + (s - pos) : at_p + s;
         if (o < capacity) {
-          idx_p[o] = e;
-          val_p[o] = a;
-          lag_p[o] = __ldg(lp + e);
+          (neg ? idx_n : idx_p)[o] = e;
+          (neg ? val_n : val_p)[o] = __ldg((neg ? vn : vp) + e);
+          (neg ? lag_n : lag_p)[o] = __ldg((neg ? ln : lp) + e);
         }
       }
-      if (kn) {
-        const long long o = on + wn + __popc(bn & below);
-        if (o < capacity) {
-          idx_n[o] = e;
-          val_n[o] = c;
-          lag_n[o] = __ldg(ln + e);
-        }
-      }
-      op += tp;
-      on += tn;
-      __syncthreads();  // s_p / s_n are reused by the next k
     }
   }
 }
 
-__global__ void __launch_bounds__(256) histogram_kernel(const float *__restrict__ vp, const float *__restrict__ vn,
-                                                         long long n, int n_hist, float delta, int *hmax,
-                                                         int *hmin) {
-  extern __shared__ int s_hist[];
-  const bool smem = n_hist <= kHistSmemMax;
-  if (smem)
-    for (int h = threadIdx.x; h < 2 * n_hist; h += blockDim.x) s_hist[h] = 0;
+// Histograms in shared memory, `rep` copies of each counter (a power of two up
+// to 32) used by lane % rep: the coefficients of a catalog fall into a few
+// bins, and a warp's 32 additions to the same few words ran one after another.
+// Four loads an array in flight a thread.  134 M pairs, 20 bins: 181 us against
+// 469 with one copy and a division a value.
+__global__ void __launch_bounds__(kHistThreads) histogram_kernel(const float *__restrict__ vp,
+                                                                 const float *__restrict__ vn, long long n,
+                                                                 int n_hist, float delta, float inv, int rep,
+                                                                 int *hmax, int *hmin) {
+  extern __shared__ int s_hist[];  // [2][n_hist][rep]; rep == 0: counted in global memory
+  for (int h = threadIdx.x; h < 2 * n_hist * rep; h += blockDim.x) s_hist[h] = 0;
   __syncthreads();
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const int hp = sparse_hist_bin(__ldg(vp + e), delta, n_hist);
-    const int hn = sparse_hist_bin(-__ldg(vn + e), delta, n_hist);
-    if (smem) {
-      atomicAdd(&s_hist[hp], 1);
-      atomicAdd(&s_hist[n_hist + hn], 1);
+  const int mine = rep ? (int)threadIdx.x & (rep - 1) : 0;
+  auto count = [&](float p, float m) {
+    const int hp = sparse_hist_bin(p, delta, inv, n_hist);
+    const int hn = sparse_hist_bin(-m, delta, inv, n_hist);
+    if (rep) {
+      atomicAdd(&s_hist[hp * rep + mine], 1);
+      atomicAdd(&s_hist[(n_hist + hn) * rep + mine], 1);
     } else {
       atomicAdd(&hmax[hp], 1);
       atomicAdd(&hmin[hn], 1);
     }
+  };
+  constexpr int U = 4;
+  const long long step = (long long)gridDim.x * kHistThreads * U;
+  long long e = (long long)blockIdx.x * kHistThreads * U + threadIdx.x;
+  for (; e + (U - 1) * kHistThreads < n; e += step) {
+    float p[U], m[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      p[k] = __ldcs(vp + e + k * kHistThreads);
+      m[k] = __ldcs(vn + e + k * kHistThreads);
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k) count(p[k], m[k]);
   }
+  for (; e < n; e += kHistThreads) count(__ldcs(vp + e), __ldcs(vn + e));  // the last, partial batch
   __syncthreads();
-  if (smem) {
-    for (int h = threadIdx.x; h < n_hist; h += blockDim.x) {
-      if (s_hist[h]) atomicAdd(&hmax[h], s_hist[h]);
-      if (s_hist[n_hist + h]) atomicAdd(&hmin[h], s_hist[n_hist + h]);
+  if (rep) {
+    for (int h = threadIdx.x; h < 2 * n_hist; h += blockDim.x) {
+      int t = 0;
+      for (int r = 0; r < rep; ++r) t += s_hist[h * rep + r];
+      if (t) atomicAdd(h < n_hist ? &hmax[h] : &hmin[h - n_hist], t);
     }
   }
+}
+
+// Workspace: the counts per CTA (at most nb CTAs, 2 nb words of 8 bytes), then
+// (where there is room) the words.
+long long compact_blocks(long long n) { return (n + kCompactBlock - 1) / kCompactBlock; }
+size_t compact_count_bytes(long long nb) { return (size_t)(2 * nb + 2) * sizeof(long long); }
+size_t compact_bytes(long long nb) {
+  return compact_count_bytes(nb) + (size_t)nb * kCompactWarps * 32 * sizeof(unsigned);
 }
 
 }  // namespace seismic
@@ -197,23 +260,27 @@ extern "C" {
 
 size_t seismic_compact_workspace_bytes(long long n_pairs) {
   if (n_pairs < 0) return 0;
-  const long long nb = (n_pairs + kCompactBlock - 1) / kCompactBlock;
-  return (size_t)(2 * nb + 2) * sizeof(long long);
+  return compact_bytes(compact_blocks(n_pairs));
 }
 
-int seismic_compact_pairs_device(const float *d_vals_pos, const int *d_lags_pos, const float *d_vals_neg,
-                                 const int *d_lags_neg, long long n_pairs, float threshold, long long capacity,
-                                 long long *d_index_pos, float *d_value_pos, int *d_lag_pos,
-                                 long long *d_index_neg, float *d_value_neg, int *d_lag_neg,
-                                 long long *d_counts, void *workspace, size_t workspace_bytes, void *stream) {
+// Both compaction calls: `count` runs the count pass, `capacity` >
+// 0 the write pass.
+static int compact_run(const float *d_vals_pos, const int *d_lags_pos, const float *d_vals_neg,
+                       const int *d_lags_neg, long long n_pairs, float threshold, long long capacity,
+                       long long *d_index_pos, float *d_value_pos, int *d_lag_pos, long long *d_index_neg,
+                       float *d_value_neg, int *d_lag_neg, long long *d_counts, void *workspace,
+                       size_t workspace_bytes, void *stream, bool count) {
   report_status(SEISMIC_OK, "");
   if (n_pairs < 0 || capacity < 0 || !(threshold >= 0.f))
     return report_status(SEISMIC_ERR_INVALID_ARGUMENT, "n_pairs, capacity and threshold must be >= 0");
-  if (!d_vals_pos || !d_lags_pos || !d_vals_neg || !d_lags_neg || !d_counts || !workspace)
+  if (!d_vals_pos || !d_lags_pos || !d_vals_neg || !d_lags_neg || (count && !d_counts) || !workspace)
     return report_status(SEISMIC_ERR_INVALID_ARGUMENT, "null buffer");
   if (capacity > 0 && (!d_index_pos || !d_value_pos || !d_lag_pos || !d_index_neg || !d_value_neg || !d_lag_neg))
     return report_status(SEISMIC_ERR_INVALID_ARGUMENT, "null output buffer with capacity > 0");
-  if (workspace_bytes < seismic_compact_workspace_bytes(n_pairs))
+  const long long nb = compact_blocks(n_pairs);
+  // a workspace with room for the block counts alone is taken too; the write
+  // pass then reads the values again
+  if (workspace_bytes < compact_count_bytes(nb))
     return report_status(SEISMIC_ERR_WORKSPACE_TOO_SMALL, "compaction workspace too small");
   int sm = 0;
   const float2 *tw;
@@ -221,27 +288,54 @@ int seismic_compact_pairs_device(const float *d_vals_pos, const int *d_lags_pos,
   int s = device_context(&sm, &tw, &ef);
   if (s) return s;
   cudaStream_t st = (cudaStream_t)stream;
-  const long long nb = (n_pairs + kCompactBlock - 1) / kCompactBlock;
   long long *counts = static_cast<long long *>(workspace);
+  unsigned *words = workspace_bytes < compact_bytes(nb) ? nullptr
+                                                        : reinterpret_cast<unsigned *>(counts + 2 * nb + 2);
+  cudaError_t e = cudaSuccess;
   if (nb == 0) {
-    cudaError_t e = cudaMemsetAsync(d_counts, 0, 2 * sizeof(long long), st);
+    if (count) e = cudaMemsetAsync(d_counts, 0, 2 * sizeof(long long), st);
     return e == cudaSuccess ? SEISMIC_OK : report_cuda(e, "compaction count clear");
   }
+  // the same grid in both passes: a CTA of the write pass owns the pairs that
+  // its count covers
   const int grid = (int)(nb < (long long)sm * 8 ? nb : (long long)sm * 8);
-  compact_count_kernel<<<grid, kCompactThreads, 0, st>>>(d_vals_pos, d_vals_neg, n_pairs, threshold, nb, counts);
-  compact_scan_kernel<<<1, 1024, 0, st>>>(counts, nb, d_counts);
-  cudaError_t e = cudaGetLastError();
+  if (count) {
+    e = cudaMemsetAsync(d_counts, 0, 2 * sizeof(long long), st);
+    if (e != cudaSuccess) return report_cuda(e, "compaction count clear");
+    compact_count_kernel<<<grid, kCompactThreads, 0, st>>>(d_vals_pos, d_vals_neg, n_pairs, threshold, nb, counts,
+                                                           words, reinterpret_cast<unsigned long long *>(d_counts));
+    e = cudaGetLastError();
+    note_launches(1);
+  }
   if (e == cudaSuccess && capacity > 0) {
     compact_write_kernel<<<grid, kCompactThreads, 0, st>>>(d_vals_pos, d_lags_pos, d_vals_neg, d_lags_neg, n_pairs,
-                                                           threshold, nb, counts, capacity, d_index_pos,
+                                                           threshold, nb, counts, words, capacity, d_index_pos,
                                                            d_value_pos, d_lag_pos, d_index_neg, d_value_neg,
                                                            d_lag_neg);
     e = cudaGetLastError();
     note_launches(1);
   }
-  if (e != cudaSuccess) return report_cuda(e, "compaction launch");
-  note_launches(2);
-  return SEISMIC_OK;
+  return e == cudaSuccess ? SEISMIC_OK : report_cuda(e, "compaction launch");
+}
+
+int seismic_compact_pairs_device(const float *d_vals_pos, const int *d_lags_pos, const float *d_vals_neg,
+                                 const int *d_lags_neg, long long n_pairs, float threshold, long long capacity,
+                                 long long *d_index_pos, float *d_value_pos, int *d_lag_pos,
+                                 long long *d_index_neg, float *d_value_neg, int *d_lag_neg,
+                                 long long *d_counts, void *workspace, size_t workspace_bytes, void *stream) {
+  return compact_run(d_vals_pos, d_lags_pos, d_vals_neg, d_lags_neg, n_pairs, threshold, capacity, d_index_pos,
+                     d_value_pos, d_lag_pos, d_index_neg, d_value_neg, d_lag_neg, d_counts, workspace,
+                     workspace_bytes, stream, true);
+}
+
+int seismic_compact_write_device(const float *d_vals_pos, const int *d_lags_pos, const float *d_vals_neg,
+                                 const int *d_lags_neg, long long n_pairs, float threshold, long long capacity,
+                                 long long *d_index_pos, float *d_value_pos, int *d_lag_pos,
+                                 long long *d_index_neg, float *d_value_neg, int *d_lag_neg,
+                                 const void *workspace, size_t workspace_bytes, void *stream) {
+  return compact_run(d_vals_pos, d_lags_pos, d_vals_neg, d_lags_neg, n_pairs, threshold, capacity, d_index_pos,
+                     d_value_pos, d_lag_pos, d_index_neg, d_value_neg, d_lag_neg, nullptr,
+                     const_cast<void *>(workspace), workspace_bytes, stream, false);
 }
 
 int seismic_histogram_device(const float *d_vals_pos, const float *d_vals_neg, long long n_pairs,
@@ -257,11 +351,15 @@ int seismic_histogram_device(const float *d_vals_pos, const float *d_vals_neg, l
   int *ef;
   int s = device_context(&sm, &tw, &ef);
   if (s) return s;
-  const long long want = (n_pairs + 255) / 256;
+  const long long want = (n_pairs + 4 * kHistThreads - 1) / (4 * kHistThreads);
   const int grid = (int)(want < (long long)sm * 8 ? want : (long long)sm * 8);
-  const size_t smem = n_classes_hist <= kHistSmemMax ? (size_t)2 * n_classes_hist * sizeof(int) : 0;
-  histogram_kernel<<<grid, 256, smem, (cudaStream_t)stream>>>(d_vals_pos, d_vals_neg, n_pairs, n_classes_hist,
-                                                             (float)(1.0 / n_classes_hist), d_max_hist, d_min_hist);
+  // copies of the counters: as many as fit the shared memory that every launch
+  // may use without an attribute; none (global counters) past kHistSmemMax bins
+  int rep = n_classes_hist <= kHistSmemMax ? 32 : 0;
+  while (rep > 1 && (size_t)2 * n_classes_hist * rep * sizeof(int) > (size_t)kHistSmemBytes) rep >>= 1;
+  const float delta = (float)(1.0 / n_classes_hist);
+  histogram_kernel<<<grid, kHistThreads, (size_t)2 * n_classes_hist * rep * sizeof(int), (cudaStream_t)stream>>>(
+      d_vals_pos, d_vals_neg, n_pairs, n_classes_hist, delta, 1.0f / delta, rep, d_max_hist, d_min_hist);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return report_cuda(e, "histogram launch");
   note_launches(1);

@@ -55,13 +55,14 @@ def histogram(vals_pos, vals_neg, n_classes_hist: int):
 
 def compact(vals_pos, lags_pos, vals_neg, lags_neg, threshold: float = 0.0) -> SparsePairs:
     """Pairs with vals_pos > threshold and vals_neg < -threshold, in packed
-    order, from packed CUDA tensors (one count pass, then the write pass)."""
+    order, from packed CUDA tensors (one count pass, then the write pass from
+    the workspace that it filled)."""
     import torch
     lib = _lib.lib()
     dev = vals_pos.device
     n = vals_pos.numel()
     ws = torch.empty(max(16, lib.seismic_compact_workspace_bytes(n)), dtype=torch.uint8, device=dev)
-    counts = torch.zeros(2, dtype=torch.int64, device=dev)
+    counts = torch.empty(2, dtype=torch.int64, device=dev)
     args = [_ptr(vals_pos), _ptr(lags_pos), _ptr(vals_neg), _ptr(lags_neg), n, ctypes.c_float(threshold)]
     _lib.check(lib.seismic_compact_pairs_device(*args, 0, None, None, None, None, None, None, _ptr(counts),
                                                 _ptr(ws), ws.numel(), _stream()))
@@ -70,8 +71,7 @@ def compact(vals_pos, lags_pos, vals_neg, lags_neg, threshold: float = 0.0) -> S
     out = [torch.empty(cap, dtype=torch.int64, device=dev), torch.empty(cap, dtype=torch.float32, device=dev),
            torch.empty(cap, dtype=torch.int32, device=dev), torch.empty(cap, dtype=torch.int64, device=dev),
            torch.empty(cap, dtype=torch.float32, device=dev), torch.empty(cap, dtype=torch.int32, device=dev)]
-    _lib.check(lib.seismic_compact_pairs_device(*args, cap, *(_ptr(t) for t in out), _ptr(counts), _ptr(ws),
-                                                ws.numel(), _stream()))
+    _lib.check(lib.seismic_compact_write_device(*args, cap, *(_ptr(t) for t in out), _ptr(ws), ws.numel(), _stream()))
     return SparsePairs(n, out[0][:cp], out[1][:cp], out[2][:cp], out[3][:cn], out[4][:cn], out[5][:cn])
 
 
