@@ -936,6 +936,32 @@ static cudaError_t launch_lag_kernel(LagArgs &a, const LagPlan &pl, const unsign
   return cudaGetLastError();
 }
 
+// j's per work item: of 32, 16, ... 1 (multiples of jp, at most `most`), the
+// largest whose busiest CTA has the least to walk: its items' j's, and a
+// twentieth of a j an item with one plane (measured: N=6000, items of 1 for items of
+// 32 cost 2.3 % where they save 2.1 % of the j's; with two planes they cost nothing).
+// The strips and the A ring run on across items.  items(jc) counts the launch's
+// items.  5 queries against 6,177 x 3 events (lags +-256) ran as 49 items of 8 on 49 of
+// 150 SMs: 198 us, 147 items of 2: 91 us.  Triangle, three products, N=4001: 12.5 ->
+// 11.9 ms; N=600 556 -> 256 us.
+template <class F>
+static int lag_item_js(int most, int jp, int nhl, long long j_rows, int sm_count, F items) {
+  int best = jp;
+  long long best_cost = -1;
+  for (int jc = 32; jc >= jp; jc >>= 1) {
+    if (jc > most || jc % jp != 0) continue;
+    const long long n = items(jc);
+    const long long grid = n < sm_count ? n : sm_count;
+    if (grid <= 0) return jc;
+    const long long cost = (n + grid - 1) / grid * (20 * (jc < j_rows ? jc : j_rows) + (nhl == 1 ? 1 : 0));
+    if (best_cost < 0 || cost < best_cost) {
+      best = jc;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
 long long lag_blocks(long long n) { return (n + kLagM - 1) / kLagM; }
 
 long long lag_block_row(long long b, long long n) { return b * kLagM < n ? b * kLagM : n; }
@@ -961,7 +987,12 @@ cudaError_t launch_lag_blocks(const void *ws, long long n, int C, int length, in
   a.L = length;
   a.shift = shift;
   a.nhl = nhl;
-  a.jc = pl.jc;
+  auto items_of = [&](int jc) {
+    long long items = 0;
+    for (long long bb = blk_begin; bb < blk_end; ++bb) items += (n - bb * kLagM + jc - 1) / jc;
+    return items;
+  };
+  a.jc = lag_item_js(pl.jc, pl.jp, nhl, n, sm_count, items_of);
   a.threshold = threshold;
   a.n_hist = n_hist;
   a.vals_pos = vp;
@@ -975,9 +1006,7 @@ cudaError_t launch_lag_blocks(const void *ws, long long n, int C, int length, in
   a.wait_probe = device_wait_probe();
   a.blk_begin = blk_begin;
   a.blk_end = blk_end;
-  long long items = 0;
-  for (long long bb = blk_begin; bb < blk_end; ++bb) items += (n - bb * kLagM + pl.jc - 1) / pl.jc;
-  return launch_lag_kernel(a, pl, xhi, xlo, n * C, items, sm_count, s);
+  return launch_lag_kernel(a, pl, xhi, xlo, n * C, items_of(a.jc), sm_count, s);
 }
 
 cudaError_t launch_lag_gemm(const float *events, long long n, int C, int length, long long ev_stride,
@@ -1001,7 +1030,10 @@ cudaError_t launch_lag_rect(const void *cat_ws, long long n_cat, const void *q_w
   LagPlan pl = lag_plan(n_cat, C, length, shift, 0, nhl);
   if (!pl.ok || col_begin < 0 || n_cols < 1 || col_begin + n_cols > n_cat || n_query < 1)
     return cudaErrorInvalidValue;
-  pl.jc = 8;  // queries per item: more items than SMs for a 64-query request (4 and 8 measured equal, 16 slower)
+  const long long nblk = (n_cols + kLagM - 1) / kLagM;
+  auto items_of = [&](int jc) { return nblk * ((n_query + jc - 1) / jc); };
+  // at most 8 queries per item (4 and 8 measured equal for a 64-query request, 16 slower)
+  pl.jc = lag_item_js(8, pl.jp, nhl, n_query, sm_count, items_of);
   if (const char *env = getenv("SEISMIC_LAG_RECT_JC")) {  // 1 .. 64, a multiple of jp
     const int v = atoi(env);
     if (v >= 1 && v <= 64 && v % pl.jp == 0) pl.jc = v;
@@ -1033,9 +1065,7 @@ cudaError_t launch_lag_rect(const void *cat_ws, long long n_cat, const void *q_w
   a.error_flag = error_flag;
   a.wait_limit = device_wait_polls();
   a.wait_probe = device_wait_probe();
-  const long long nblk = (n_cols + kLagM - 1) / kLagM;
-  const long long items = nblk * ((n_query + pl.jc - 1) / pl.jc);
-  return launch_lag_kernel(a, pl, a.xhi, a.xlo, n_cat * C, items, sm_count, s);
+  return launch_lag_kernel(a, pl, a.xhi, a.xlo, n_cat * C, items_of(pl.jc), sm_count, s);
 }
 
 }  // namespace seismic
