@@ -429,7 +429,12 @@ template <int RL> __host__ __device__ constexpr uint32_t scan_block_bits(int b) 
   return m;
 }
 
-template <int P, bool VOTE>
+// STRAIGHT: the lag search straight through a thread's values (all owners of a
+// warp in step), else block by block.  The staged form searches straight: ms,
+// blocks / straight, P=1024 5.99 / 5.86, Q=1024 x 2 frames of three channels 10.39 /
+// 10.04, Q=512 x 4 17.61 / 17.47, P=4096 13.44 / 13.00, P=2048 12.56 / 12.63.  The direct
+// form by blocks: P=256 2.04 / 2.07, P=8192 6.39 / 7.36 (three channels 8.7 / 12.4), the batch 34.2 / 35.3.
+template <int P, bool VOTE, bool STRAIGHT>
 __device__ __forceinline__ void scan_and_write(const PairArgs &a, float2 (&v)[32], long long ia, long long ja,
                                                long long ib, long long jb, bool out_b, int t, int g, unsigned *red,
                                                int *hist, bool smem_hist, uint32_t wmask, float2 *xbuf) {
@@ -518,28 +523,57 @@ __device__ __forceinline__ void scan_and_write(const PairArgs &a, float2 (&v)[32
     }
   }
   // ---- phase C: threads holding a winning value find its smallest lag
-  //      (first occurrence in increasing lag, as the reference's scan), in
-  //      the blocks that hold it: a bit per winning value, then the lags of
-  //      the set bits (one, but for ties)
+  //      (first occurrence in increasing lag, as the reference's scan): a bit
+  //      per value equal to it, then the lags of the set bits (one, but for ties)
   int lag[4] = {INT_MAX, INT_MAX, INT_MAX, INT_MAX};
+  auto smallest_lag = [&](uint32_t hits) {
+    int l = INT_MAX;
+    while (hits) {
+      const int e = __ffs(hits) - 1;
+      hits &= hits - 1;
+      const int m = t + (e / RL) * G + (e % RL) * (P / RL);
+      l = min(l, d0 + ((m - d0) & (P - 1)));
+    }
+    return l;
+  };
+  if constexpr (STRAIGHT) {
+    // a round takes one result of every owner at once, straight through the 32
+    // values whichever series it is of; a thread that holds several goes round again
+    unsigned todo = 0;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if (key[k] != 0 && own[k] == key[k]) {
-      const float x = __uint_as_float(key[k] | ((k & 1) ? 0x80000000u : 0u));
-      uint32_t hits = 0;
+    for (int k = 0; k < 4; ++k)
+      if (key[k] != 0 && own[k] == key[k]) todo |= 1u << k;
+    while (todo) {
+      const int k = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const unsigned bits =
+          (k & 2 ? (k & 1 ? key[3] : key[2]) : (k & 1 ? key[1] : key[0])) | ((unsigned)(k & 1) << 31);
+      const float none = __int_as_float(0x7fc00000);  // equals nothing
+      const float wx = k < 2 ? __uint_as_float(bits) : none, wy = k < 2 ? none : __uint_as_float(bits);
+      uint32_t part[4] = {0, 0, 0, 0};
 #pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        if (blk[k][b] == x) {
+      for (int e = 0; e < 32; ++e)
+        if (v[e].x == wx || v[e].y == wy) part[e & 3] |= 1u << e;
+      const int l = smallest_lag((part[0] | part[1] | part[2] | part[3]) & wmask);
 #pragma unroll
-          for (int e = 0; e < 32; ++e)
-            if (in_scan_block<RL>(e, b) && (k < 2 ? v[e].x : v[e].y) == x) hits |= 1u << e;
+      for (int h = 0; h < 4; ++h)
+        if (k == h) lag[h] = l;
+    }
+  } else {  // result by result, in the blocks that hold it
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (key[k] != 0 && own[k] == key[k]) {
+        const float x = __uint_as_float(key[k] | ((k & 1) ? 0x80000000u : 0u));
+        uint32_t hits = 0;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          if (blk[k][b] == x) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+              if (in_scan_block<RL>(e, b) && (k < 2 ? v[e].x : v[e].y) == x) hits |= 1u << e;
+          }
         }
-      }
-      while (hits) {
-        const int e = __ffs(hits) - 1;
-        hits &= hits - 1;
-        const int m = t + (e / RL) * G + (e % RL) * (P / RL);
-        lag[k] = min(lag[k], d0 + ((m - d0) & (P - 1)));
+        lag[k] = smallest_lag(hits);
       }
     }
   }
