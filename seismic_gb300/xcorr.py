@@ -74,18 +74,23 @@ def xcorr(events, shift: int, threshold: float = 0.0, n_classes_hist: int = 0, p
         lp = torch.empty(m, dtype=torch.int32, device=dev)
         vn = torch.empty(m, dtype=torch.float32, device=dev)
         ln = torch.empty(m, dtype=torch.int32, device=dev)
-        hmax = torch.zeros(max(n_classes_hist, 1), dtype=torch.int32, device=dev)
-        hmin = torch.zeros(max(n_classes_hist, 1), dtype=torch.int32, device=dev)
+        # both histograms cleared by one fill (none without histograms): each fill
+        # is a launch, and a small call is bound by this function's own work
+        hist = torch.zeros(2 * max(n_classes_hist, 0), dtype=torch.int32, device=dev)
+        hmax, hmin = hist[:max(n_classes_hist, 0)], hist[max(n_classes_hist, 0):]
         s = stream if stream is not None else torch.cuda.current_stream(dev)
         ws_ptr, ws_bytes = (None, 0) if workspace is None else (workspace.data_ptr(),
                                                                   workspace.numel() * workspace.element_size())
-        with torch.cuda.device(dev):
-            st = lib.seismic_xcorr_device(ev.data_ptr(), n, c, length, c * length, length, padded_size, shift,
-                                          float(threshold), n_classes_hist, f, vp.data_ptr(), lp.data_ptr(),
-                                          vn.data_ptr(), ln.data_ptr(), hmax.data_ptr(), hmin.data_ptr(),
-                                          ws_ptr, ws_bytes, ctypes.c_void_p(s.cuda_stream))
+        args = (ev.data_ptr(), n, c, length, c * length, length, padded_size, shift, float(threshold), n_classes_hist,
+                f, vp.data_ptr(), lp.data_ptr(), vn.data_ptr(), ln.data_ptr(), hmax.data_ptr(), hmin.data_ptr(), ws_ptr,
+                ws_bytes, s.cuda_stream)
+        if dev.index == torch.cuda.current_device():
+            st = lib.seismic_xcorr_device(*args)
+        else:
+            with torch.cuda.device(dev):
+                st = lib.seismic_xcorr_device(*args)
         _lib.check(st)
-        return XcorrResult(vp, lp, vn, ln, hmax[:n_classes_hist], hmin[:n_classes_hist])
+        return XcorrResult(vp, lp, vn, ln, hmax, hmin)
 
     ev = np.ascontiguousarray(events, dtype=np.float32)
     n, c, length = _shape3(ev)
