@@ -170,22 +170,23 @@ template <int P> __device__ __forceinline__ void spectra_body(const SpectraArgs 
   }
   group_sum_pair<G>(eah, eal, red, g, t);
   group_sum_pair<G>(ebh, ebl, red, g, t);
-  // FP64 once per group: norms, inverse norms rounded once, and the
-  // spectrum scale factors, handed to the group through `red`
-  if (t == 0) {
-    const double na = sqrt(ldexp((double)eah + (double)eal, 2 * xea));
-    const double nb = sqrt(ldexp((double)ebh + (double)ebl, 2 * xeb));
-    const double ia = na > 0.0 ? 1.0 / na : 0.0;
-    const double ib = nb > 0.0 ? 1.0 / nb : 0.0;
-    a.norms[row_a] = na;
-    a.inv_norms[row_a] = split_double(ia);
-    if (has_b) {
-      a.norms[row_b] = nb;
-      a.inv_norms[row_b] = split_double(ib);
+  // FP64 once per row: norms, inverse norms rounded once, and the spectrum
+  // scale factors, handed to the group through `red`.  Threads 0 and 1 take a
+  // row each, from thread 0's sums (a sum's low part depends on the thread):
+  // one FP64 square root and division on the path instead of two.
+  {
+    const int lane0 = G < 32 ? (int)(threadIdx.x & 31) & ~(G - 1) : 0;
+    const float bh = __shfl_sync(group_lane_mask<G>(), ebh, lane0), bl = __shfl_sync(group_lane_mask<G>(), ebl, lane0);
+    if (t < 2) {
+      const double e = t == 0 ? (double)eah + (double)eal : (double)bh + (double)bl;
+      const double nrm = sqrt(ldexp(e, 2 * (t == 0 ? xea : xeb)));
+      const double inv = nrm > 0.0 ? 1.0 / nrm : 0.0;
+      if (t == 0 || has_b) {
+        a.norms[row_a + t] = nrm;
+        a.inv_norms[row_a + t] = split_double(inv);
+      }
+      reinterpret_cast<float *>(red)[t] = a.prescale ? (float)inv : 1.f;
     }
-    float *scale = reinterpret_cast<float *>(red);
-    scale[0] = a.prescale ? (float)ia : 1.f;
-    scale[1] = a.prescale ? (float)ib : 1.f;
   }
   group_sync<G>(g);
 
