@@ -58,9 +58,9 @@ namespace seismic {
 constexpr int kStagedHistMax = 1024;  // larger histograms use global atomics
 constexpr int kStagedRingMax = 16;
 // Decoded items published by the producer; it runs at most kStagedRingMax
-// units (>= 2 per item) ahead of the slowest FFT thread, so 16 entries never
+// units (>= 1 per item) ahead of the slowest FFT thread, so 32 entries never
 // wrap onto an item still being read.
-constexpr int kItemRing = 16;
+constexpr int kItemRing = 32;
 constexpr size_t kStagedSmemBudget = 227 * 1024;
 
 template <int P, int NWARP, int RU, int ST> struct Staged {  // RU: chunks r per ring slot, ST: spectra type
@@ -85,10 +85,6 @@ template <int P, int NWARP, int RU, int ST> struct Staged {  // RU: chunks r per
   // are half as long and gain nothing from a deeper ring (FP16 Q=512 x 4 17.28 / 17.39).
   static constexpr bool SPLIT_EX = ST == 0;
   static constexpr int EX_LEN = SPLIT_EX ? padded_len<P / 2>() : padded_len<P>();
-  // A unit's barrier is polled while the one before it is multiplied: hides the
-  // poll behind the half types' longer products (FP16 Q=1024 x 2, three channels, N=1733
-  // 3.37 / 3.16 ms), costs FP32 1-3 % (Q=512 x 4 17.6 / 17.9).
-  static constexpr bool EARLY_POLL = ST != 0;
   static constexpr size_t EX_BYTES = (size_t)NG * EX_LEN * sizeof(float2);
   static constexpr size_t RED_BYTES = (size_t)NG * NW * 8 * sizeof(unsigned);
   static constexpr size_t PROD_OFF = (EX_BYTES + RED_BYTES + 15) / 16 * 16;
@@ -349,11 +345,11 @@ __global__ void __launch_bounds__(NWARP * 32 + 32, 1)
       CoupleAcc y;
       y.zero();
       // units of the item; a warp releases a slot with one arrive
-      bool ready = true;  // the first unit's wait is above
       for (int c = 0; c < C && !stop; ++c) {
 #pragma unroll
         for (int rp = 0; rp < 8; rp += RU) {
-          if (!__all_sync(0xffffffffu, ready) && !consumer_wait_warp(&full[slot], phase, s_abort)) {
+          // (the first unit's wait is above)
+          if ((c > 0 || rp > 0) && !consumer_wait_warp(&full[slot], phase, s_abort)) {
             stop = true;
             break;
           }
@@ -362,11 +358,6 @@ __global__ void __launch_bounds__(NWARP * 32 + 32, 1)
           if (++slot == K) {
             slot = 0;
             phase ^= 1u;
-          }
-          if constexpr (SH::EARLY_POLL) {
-            if (rp + RU < 8 || c + 1 < C) ready = tc::mbar_test_wait(&full[slot], phase);
-          } else {
-            ready = false;
           }
 #pragma unroll
           for (int h = 0; h < RU; ++h) {
@@ -419,14 +410,15 @@ constexpr int staged_wide_warps(int P) { return P >= 4096 ? 12 : (P == 2048 ? 14
 
 // CTA shape of a launch: FFT warps per CTA and chunks per ring slot.  In
 // order: a shape the autotuner forces while timing, SEISMIC_STAGED_WARPS
-// ("12", "wide") / SEISMIC_STAGED_RU ("2", "4"), the tuner's cached choice
+// ("12", "wide") / SEISMIC_STAGED_RU ("2", "4", "8"), the tuner's cached choice
 // for exactly (P, spectrum rows), else the built-in rule: the wide CTA (the
-// most FFT warps that keep 128 registers a thread) with 4-chunk slots.
+// most FFT warps that keep 128 registers a thread) with the longest slots that
+// launch_staged_p's rule takes (8 or 4 chunks).
 // Measured with items of TI x TJ events, FP32, M pairs/s, 12 warps / wide:
 // overlap-save Q=512 x 4 rows 710 / 825, Q=1024 x 2 rows 451 / 516, P=512
 // one channel 977 / 1128, P=1024 523 / 585, P=1024 three channels 380 /
 // 469, P=2048 219 / 274, P=2048 three channels 192 / 195 (P=4096: the same
-// CTA).  Half-precision spectra always take 4-chunk slots; an FP32 launch
+// CTA).  Half-precision spectra take no 2-chunk slots; an FP32 launch
 // whose item rows leave no room for two 4-chunk slots takes 2
 // (launch_staged_p).
 struct StagedShape {
@@ -434,7 +426,7 @@ struct StagedShape {
 };
 static StagedShape staged_shape(int P, const PairArgs &a) {
   const int rows = spectrum_rows(a);
-  int w = a.staged_warps, ru = a.staged_ru;
+  int w = a.staged_warps, ru = a.staged_ru == 4 ? 8 : a.staged_ru;  // the tuner times 2 chunks against the rule's
   if (!w) {
     const char *e = getenv("SEISMIC_STAGED_WARPS");
     if (e && strcmp(e, "wide") == 0) w = staged_wide_warps(P);
@@ -444,15 +436,17 @@ static StagedShape staged_shape(int P, const PairArgs &a) {
     const char *e = getenv("SEISMIC_STAGED_RU");
     if (e && strcmp(e, "2") == 0) ru = 2;
     if (e && strcmp(e, "4") == 0) ru = 4;
+    if (e && strcmp(e, "8") == 0) ru = 8;
   }
   int tw = 0, tru = 0;
   if ((!w || !ru) && tune_staged_lookup(P, rows, &tw, &tru)) {
     if (!w) w = tw;
-    if (!ru) ru = tru;
+    if (!ru) ru = tru == 2 ? 2 : 0;
   }
   if (!w) w = staged_wide_warps(P);
   w = (w == kStagedWarps) ? kStagedWarps : staged_wide_warps(P);
-  ru = (a.stype != 0 || ru != 2) ? 4 : 2;
+  if (ru == 0) ru = 8;
+  if (a.stype != 0 && ru == 2) ru = 4;
   return StagedShape{w, ru};
 }
 
@@ -571,14 +565,31 @@ template <int P> static cudaError_t launch_staged_p(const PairArgs &a, int sm_co
   const bool wide = sh.nwarp == WW;
   // the default CTA with its default item geometry: the compile-time form
   const bool ct = wide && staged_item_rows(WW * 32 / (P / 32), a) == KT;
+  // The default slot: all eight chunks of a spectrum row, where the ring holds
+  // three such slots, or two and an event has one row.  Every unit costs its
+  // wait, vote and arrive: 2-chunk slots run 6-21 % slower than 4-chunk ones,
+  // 8-chunk ones faster still (ms, 4 / 8 chunks): Q=512 x 4 17.46 / 16.35, FP16
+  // 17.06 / 15.77, Q=1024 x 2 frames of three channels 10.03 / 9.81, P=1024 with three
+  // channels 5.35 / 5.15, P=2048 12.61 / 11.90 (with three channels, two slots, 7.43 / 7.51: four).
+  if constexpr (P <= 2048) {
+    auto fits = [&](int k) { return k >= 3 || (k == 2 && spectrum_rows(a) == 1); };
+    if (ct && sh.ru == 8) {
+      if (a.stype == 0 && fits(staged_ring_slots<P, WW, 8, 0>(a, nullptr)))
+        return launch_staged_t<P, WW, 8, 0, KT>(a, sm_count, s);
+      if (a.stype == 1 && fits(staged_ring_slots<P, WW, 8, 1>(a, nullptr)))
+        return launch_staged_t<P, WW, 8, 1, KT>(a, sm_count, s);
+      if (a.stype == 2 && fits(staged_ring_slots<P, WW, 8, 2>(a, nullptr)))
+        return launch_staged_t<P, WW, 8, 2, KT>(a, sm_count, s);
+    }
+  }
   switch (a.stype) {
     case 0:
       if (wide) {
-        if (sh.ru == 4 && staged_ring_slots<P, WW, 4, 0>(a, nullptr) >= 2)
+        if (sh.ru != 2 && staged_ring_slots<P, WW, 4, 0>(a, nullptr) >= 2)
           return ct ? launch_staged_t<P, WW, 4, 0, KT>(a, sm_count, s) : launch_staged_t<P, WW, 4, 0, 0>(a, sm_count, s);
         return launch_staged_t<P, WW, 2, 0, 0>(a, sm_count, s);
       }
-      return (sh.ru == 4 && staged_ring_slots<P, kStagedWarps, 4, 0>(a, nullptr) >= 2)
+      return (sh.ru != 2 && staged_ring_slots<P, kStagedWarps, 4, 0>(a, nullptr) >= 2)
                  ? launch_staged_t<P, kStagedWarps, 4, 0, 0>(a, sm_count, s)
                  : launch_staged_t<P, kStagedWarps, 2, 0, 0>(a, sm_count, s);
     case 1:
