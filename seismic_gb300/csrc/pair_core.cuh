@@ -405,11 +405,13 @@ template <int P> __device__ __forceinline__ uint32_t window_mask(int t, int shif
 // What bounded it: clock counts put 35-44 % of the FFT threads' time here (the
 // search for the winners' lags 15-23 %, the epilogue 3-15 %, most of it
 // IEEE divisions on one thread).  So the search looks only into the block of
-// eight values that holds a winner, four threads finish one result each, and no
-// division is left.  With the packed arithmetic of fft_core.cuh, ms before /
-// after (FP32, full lag window, N=3000 but N=2000 at P=4096): P=256 2.42 / 2.03, P=512
-// 4.18 / 3.29, P=1024 8.02 / 6.06, P=2048 16.7 / 13.4, P=4096 20.7 / 14.0, with three
-// channels 18.9 / 16.2; overlap-save Q=512 x 4 (N=6000) 20.5 / 18.4.
+// eight values that holds a winner, or goes straight through the values with
+// every owner of the warp in step, four threads finish one result each, and no
+// division is left.  With the packed arithmetic of fft_core.cuh and the ring of
+// staged_core.cuh, ms before / now (FP32, full lag window, N=3000 but N=2000 at
+// P=4096): P=256 2.42 / 2.04, P=512 4.18 / 3.09, P=1024 8.02 / 5.77, P=2048 16.7 / 11.9,
+// P=4096 20.7 / 13.0, with three channels 18.9 / 16.1; overlap-save Q=512 x 4 (N=6000)
+// 20.5 / 16.2.
 
 // Prescaled liveness by the copy-and-vote path of scan_and_write (VOTE), or
 // by thread 0's loads in the epilogue.  Measured, M pairs/s, vote vs loads:

@@ -414,10 +414,10 @@ constexpr int staged_wide_warps(int P) { return P >= 4096 ? 12 : (P == 2048 ? 14
 // for exactly (P, spectrum rows), else the built-in rule: the wide CTA (the
 // most FFT warps that keep 128 registers a thread) with the longest slots that
 // launch_staged_p's rule takes (8 or 4 chunks).
-// Measured with items of TI x TJ events, FP32, M pairs/s, 12 warps / wide:
-// overlap-save Q=512 x 4 rows 710 / 825, Q=1024 x 2 rows 451 / 516, P=512
-// one channel 977 / 1128, P=1024 523 / 585, P=1024 three channels 380 /
-// 469, P=2048 219 / 274, P=2048 three channels 192 / 195 (P=4096: the same
+// Measured with items of TI x TJ events, FP32, ms, 12 warps / wide:
+// overlap-save Q=512 x 4 rows (N=6000) 20.2 / 17.5, Q=1024 x 2 frames of three
+// channels (N=3000) 12.3 / 10.0, P=512 (N=3000) 3.50 / 3.23, P=1024 6.25 / 5.86, P=2048 with
+// three channels (N=2000) 8.25 / 7.44 (P=4096: the same
 // CTA).  Half-precision spectra take no 2-chunk slots; an FP32 launch
 // whose item rows leave no room for two 4-chunk slots takes 2
 // (launch_staged_p).
