@@ -186,7 +186,8 @@ __global__ void __launch_bounds__(kCompactThreads) compact_write_kernel(
         const long long e = (q * kCompactWords + (k & (kCompactWords - 1))) * 32 + bit;
         const bool neg = s >= pos;
         const long long o = neg ? at_n + (s - pos) : at_p + s;
-        if (o < capacity) {
+        // (e and o lie in range whenever the counts and words are those of these arrays)
+        if (e < n && o >= 0 && o < capacity) {
           (neg ? idx_n : idx_p)[o] = e;
           (neg ? val_n : val_p)[o] = __ldg((neg ? vn : vp) + e);
           (neg ? lag_n : lag_p)[o] = __ldg((neg ? ln : lp) + e);
