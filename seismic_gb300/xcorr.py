@@ -5,7 +5,11 @@ events of one catalog and returns the packed upper-triangle outputs.
 
 * numpy input  -> ``seismic_xcorr_host`` (copies in, runs, copies back);
 * torch CUDA tensor input -> ``seismic_xcorr_device`` on torch's current
-  stream, outputs are CUDA tensors (nothing leaves the device).
+  stream, outputs are CUDA tensors (nothing leaves the device).  With
+  ``stream=`` the whole call (a copy of strided events, the histograms' clear,
+  the kernels) runs on that stream and nothing on the current one; as with
+  any CUDA op the caller orders the two (``wait_stream``) for events that
+  another stream still writes and before reading the outputs elsewhere.
 
 events are float32 shaped (N, L) or (N, C, L); with C > 1 the coefficient
 series is the mean over channels of the per-channel normalised series.
@@ -54,6 +58,35 @@ def _shape3(events):
     raise ValueError("events must be (N, L) or (N, C, L)")
 
 
+def _xcorr_cuda(lib, events, shift, threshold, n_classes_hist, padded_size, f, workspace, cuda_stream) -> XcorrResult:
+    """Allocations, the histograms' clear and the kernels on torch's current stream, whose handle is `cuda_stream`."""
+    import torch
+    ev = events.contiguous()
+    n, c, length = _shape3(ev)
+    m = n_pairs(n)
+    dev = ev.device
+    vp = torch.empty(m, dtype=torch.float32, device=dev)
+    lp = torch.empty(m, dtype=torch.int32, device=dev)
+    vn = torch.empty(m, dtype=torch.float32, device=dev)
+    ln = torch.empty(m, dtype=torch.int32, device=dev)
+    # both histograms cleared by one fill (none without histograms): each fill
+    # is a launch, and a small call is bound by this function's own work
+    hist = torch.zeros(2 * max(n_classes_hist, 0), dtype=torch.int32, device=dev)
+    hmax, hmin = hist[:max(n_classes_hist, 0)], hist[max(n_classes_hist, 0):]
+    ws_ptr, ws_bytes = (None, 0) if workspace is None else (workspace.data_ptr(),
+                                                              workspace.numel() * workspace.element_size())
+    args = (ev.data_ptr(), n, c, length, c * length, length, padded_size, shift, float(threshold), n_classes_hist,
+            f, vp.data_ptr(), lp.data_ptr(), vn.data_ptr(), ln.data_ptr(), hmax.data_ptr(), hmin.data_ptr(), ws_ptr,
+            ws_bytes, cuda_stream)
+    if dev.index == torch.cuda.current_device():
+        st = lib.seismic_xcorr_device(*args)
+    else:
+        with torch.cuda.device(dev):
+            st = lib.seismic_xcorr_device(*args)
+    _lib.check(st)
+    return XcorrResult(vp, lp, vn, ln, hmax, hmin)
+
+
 def xcorr(events, shift: int, threshold: float = 0.0, n_classes_hist: int = 0, padded_size: int = 0,
           form: str = "fp32", stream=None, workspace=None) -> XcorrResult:
     lib = _lib.lib()
@@ -66,31 +99,22 @@ def xcorr(events, shift: int, threshold: float = 0.0, n_classes_hist: int = 0, p
     if is_torch:
         if not events.is_cuda or events.dtype != torch.float32:
             raise ValueError("torch events must be a float32 CUDA tensor")
-        ev = events.contiguous()
-        n, c, length = _shape3(ev)
-        m = n_pairs(n)
-        dev = ev.device
-        vp = torch.empty(m, dtype=torch.float32, device=dev)
-        lp = torch.empty(m, dtype=torch.int32, device=dev)
-        vn = torch.empty(m, dtype=torch.float32, device=dev)
-        ln = torch.empty(m, dtype=torch.int32, device=dev)
-        # both histograms cleared by one fill (none without histograms): each fill
-        # is a launch, and a small call is bound by this function's own work
-        hist = torch.zeros(2 * max(n_classes_hist, 0), dtype=torch.int32, device=dev)
-        hmax, hmin = hist[:max(n_classes_hist, 0)], hist[max(n_classes_hist, 0):]
-        s = stream if stream is not None else torch.cuda.current_stream(dev)
-        ws_ptr, ws_bytes = (None, 0) if workspace is None else (workspace.data_ptr(),
-                                                                  workspace.numel() * workspace.element_size())
-        args = (ev.data_ptr(), n, c, length, c * length, length, padded_size, shift, float(threshold), n_classes_hist,
-                f, vp.data_ptr(), lp.data_ptr(), vn.data_ptr(), ln.data_ptr(), hmax.data_ptr(), hmin.data_ptr(), ws_ptr,
-                ws_bytes, s.cuda_stream)
-        if dev.index == torch.cuda.current_device():
-            st = lib.seismic_xcorr_device(*args)
-        else:
-            with torch.cuda.device(dev):
-                st = lib.seismic_xcorr_device(*args)
-        _lib.check(st)
-        return XcorrResult(vp, lp, vn, ln, hmax, hmin)
+        args = (lib, events, shift, threshold, n_classes_hist, padded_size, f, workspace)
+        current = torch.cuda.current_stream(events.device)
+        if stream is None or stream.cuda_stream == current.cuda_stream:
+            return _xcorr_cuda(*args, current.cuda_stream)
+        side = stream if isinstance(stream, torch.cuda.Stream) else torch.cuda.ExternalStream(stream.cuda_stream,
+                                                                                             device=events.device)
+        with torch.cuda.stream(side):
+            r = _xcorr_cuda(*args, side.cuda_stream)
+        # inputs are read on `side`, outputs (allocated there) may be read here:
+        # neither's memory is handed out again before the other stream is done
+        for t in (events, workspace):
+            if isinstance(t, torch.Tensor) and t.is_cuda:
+                t.record_stream(side)
+        for t in (r.vals_pos, r.lags_pos, r.vals_neg, r.lags_neg, r.max_hist):
+            t.record_stream(current)
+        return r
 
     ev = np.ascontiguousarray(events, dtype=np.float32)
     n, c, length = _shape3(ev)
