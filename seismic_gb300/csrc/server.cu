@@ -581,6 +581,9 @@ extern "C" int seismic_server_create(const float *catalog, long long n_catalog, 
   const size_t per_req = request_bytes(s, max_query_events, n_catalog);
   s->pool_bytes = hbm_budget_bytes ? round256(hbm_budget_bytes) : per_req * (size_t)n_slots;
   if (e == cudaSuccess) e = cudaMalloc(&s->pool, s->pool_bytes);
+  // the top-K kernel's shared memory: without it every request would fail at its launch
+  if (e == cudaSuccess && topk > 0)
+    e = ensure_dynamic_smem((const void *)topk_kernel, kTopKBuffer * (int)sizeof(unsigned long long));
   if (e != cudaSuccess) {
     cudaFree(s->cat_spectra);
     cudaFree(s->cat_norms);
@@ -595,8 +598,7 @@ extern "C" int seismic_server_create(const float *catalog, long long n_catalog, 
   s->slot_busy.assign(n_slots, false);
   for (auto &st : s->streams) cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
   for (auto &ev : s->pair_done) cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-  // make sure the kernels' attributes are set before concurrent use
-  ensure_dynamic_smem((const void *)topk_kernel, kTopKBuffer * (int)sizeof(unsigned long long));
+  // make sure the pair kernel's attributes are set before concurrent use
   pair_ctas_per_sm(P);
   int dev = 0;
   cudaGetDevice(&dev);
