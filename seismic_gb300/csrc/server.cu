@@ -49,16 +49,24 @@ namespace seismic {
 // One CTA per query row: the K largest values of vals[row][0..n) (ties to the
 // smaller column), as (value, catalog index = col_begin + column).
 //
-// Two passes over the row.  The first takes the maxima of 64 interleaved
-// sixteenths of a warp; the K-th largest of them bounds the K-th largest value
-// from below.  The second collects the values at or above the bound, a batch of
-// kTopKBatch columns at a time and in column order, and sorts what it has down to
-// the K best whenever the buffer may overflow (from then on only larger values
-// enter: later columns lose ties).  On coefficients a few dozen values pass the
-// bound, so there is one small sort.  What bounds it: the latency of the
-// row's loads, 4 to 8 in flight a thread.  50,000 columns, K = 16: 19 us for
+// Two passes over the row.  The first takes the maxima of 64 interleaved groups
+// of 16 lanes (half a warp); the K-th largest of them bounds the K-th largest
+// value from below.  The second collects the values at or above the bound, a
+// batch of kTopKBatch columns at a time and in column order, and sorts what it
+// has down to the K best whenever the buffer may overflow (from then on only
+// larger values enter: later columns lose ties).  On coefficients a few dozen
+// values pass the bound, so there is one small sort.  What bounds it: the
+// latency of the row's loads, 4 to 8 in flight a thread.  50,000 columns, K = 16: 19 us for
 // 64 rows against 300 for a sorted list a thread in local memory and K rounds
 // of an arg-max over the CTA; 6,177 columns, 5 rows: 8.5 against 44.
+//
+// Ties.  Of the values equal to the bound only the first K can be among the K
+// best, but on a row that the threshold has cut to zeros the bound is 0 and
+// all of a batch passes.  A first batch of which far more than K pass (8 K:
+// rows without ties stay below) is therefore collected again with its ties
+// ranked in column order and cut at K; if it holds K, later columns must exceed
+// the bound.  64 rows of zeros, K = 16: 20 us for 50,000 columns (49 without this, 57
+// for the lists a thread), 10.5 for 6,177 (41, 21).
 constexpr int kTopKMax = 64;
 constexpr int kTopKThreads = 1024;
 constexpr int kTopKGroups = 64;                             // groups of kTopKThreads / 64 lanes
@@ -102,6 +110,8 @@ __global__ void __launch_bounds__(kTopKThreads)
   __shared__ float s_max[kTopKGroups];
   __shared__ float s_bound;
   __shared__ int s_count;
+  __shared__ int s_ties[4][32];  // the first batch's values equal to the bound, by quarter and warp
+  static_assert(kTopKThreads == 32 * 32, "one lane per warp's count");
   const long long row = blockIdx.x;
   const float *v = vals + row * n;
   constexpr int GL = kTopKThreads / kTopKGroups;  // lanes per group
@@ -131,7 +141,7 @@ __global__ void __launch_bounds__(kTopKThreads)
     if (rank == k - 1) s_bound = mine;  // k <= kTopKGroups
   }
   __syncthreads();
-  const float bound = s_bound;
+  float bound = s_bound;
 
   // ---- candidates in column order
   unsigned long long last = 0;  // the K-th best key once K are sorted: later columns must beat its value
@@ -142,21 +152,46 @@ __global__ void __launch_bounds__(kTopKThreads)
       const long long c = j0 + q * kTopKThreads + threadIdx.x;
       x[q] = c < n ? __ldg(v + c) : -INFINITY;
     }
+    auto collect = [&]() {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const long long c = j0 + q * kTopKThreads + threadIdx.x;
-      const unsigned long long key = topk_key(x[q], (unsigned)c);
-      const bool take = c < n && x[q] >= bound && key > last;
-      const unsigned votes = __ballot_sync(0xffffffffu, take);
-      if (votes) {  // uniform over the warp
-        int at = 0;
-        if (lane == __ffs(votes) - 1) at = atomicAdd(&s_count, __popc(votes));
-        at = __shfl_sync(0xffffffffu, at, __ffs(votes) - 1);
-        if (take) buf[at + __popc(votes & ((1u << lane) - 1u))] = key;
+      for (int q = 0; q < 4; ++q) {
+        const long long c = j0 + q * kTopKThreads + threadIdx.x;
+        const unsigned long long key = topk_key(x[q], (unsigned)c);
+        const bool take = c < n && x[q] >= bound && key > last;
+        const unsigned votes = __ballot_sync(0xffffffffu, take);
+        if (votes) {  // uniform over the warp
+          int at = 0;
+          if (lane == __ffs(votes) - 1) at = atomicAdd(&s_count, __popc(votes));
+          at = __shfl_sync(0xffffffffu, at, __ffs(votes) - 1);
+          if (take) buf[at + __popc(votes & ((1u << lane) - 1u))] = key;
+        }
       }
+      __syncthreads();
+    };
+    collect();
+    int have = s_count;
+    if (j0 == 0 && have > 8 * k) {  // uniform over the CTA
+      int rank[4], ties = 0;  // of this thread's values among those equal to the bound
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const unsigned eq = __ballot_sync(0xffffffffu, q * kTopKThreads + threadIdx.x < n && x[q] == bound);
+        rank[q] = __popc(eq & ((1u << lane) - 1u));
+        if (lane == 0) s_ties[q][threadIdx.x >> 5] = __popc(eq);
+      }
+      __syncthreads();  // (everyone has read s_count too)
+      if (threadIdx.x == 0) s_count = 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const unsigned cnt = (unsigned)s_ties[q][lane];
+        rank[q] += ties + (int)__reduce_add_sync(0xffffffffu, lane < (int)(threadIdx.x >> 5) ? cnt : 0u);
+        ties += (int)__reduce_add_sync(0xffffffffu, cnt);
+        if (x[q] == bound && rank[q] >= k) x[q] = __int_as_float(0x7fc00000);  // NaN: not taken
+      }
+      __syncthreads();
+      collect();
+      have = s_count;
+      if (ties >= k) bound = nextafterf(bound, INFINITY);  // later columns: only larger values
     }
-    __syncthreads();
-    const int have = s_count;
     const bool end = j0 + kTopKBatch >= n;
     if (have > kTopKSlack || end) {  // sort what there is; only the K best stay
       int p2 = 2;
