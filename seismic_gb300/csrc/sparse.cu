@@ -19,6 +19,7 @@
 // the values' bytes, and touches only the kept pairs.  Output order is the
 // packed order.
 #include <cstdint>
+#include <type_traits>
 
 #include "../../include/seismic_gb300.h"
 #include "kernels.cuh"
@@ -32,6 +33,11 @@ void note_launches(unsigned n);
 constexpr int kCompactThreads = 256;
 constexpr int kCompactWarps = kCompactThreads / 32;
 constexpr int kCompactWords = 16;                                     // 32-pair words a warp and side
+// Kept pairs of a chunk's 1024 (both sides) from which its 32 words are gone
+// through one by one, a bit a lane, instead of finding each round's pairs (16 rounds
+// of the search cost what 32 words do: 16.8 M pairs, all kept, 262 us by
+// search and 201 by words; a fifth kept 102.5 and, from 256 on by words, 106).
+constexpr int kCompactDense = 512;
 constexpr int kCompactBlock = kCompactWarps * kCompactWords * 32;     // pairs per block
 constexpr int kHistThreads = 256;
 constexpr int kHistSmemMax = 4096;
@@ -82,6 +88,15 @@ __device__ __forceinline__ unsigned compact_word(const float *__restrict__ vp, c
   return word;
 }
 
+// The CTA's sum of a number a warp.  (A 64-bit shared atomicAdd a thread is a
+// loop that 256 threads run one after another: 8 us of a small call.)
+__device__ __forceinline__ long long warps_sum(const long long (&v)[kCompactWarps]) {
+  long long t = 0;
+#pragma unroll
+  for (int w = 0; w < kCompactWarps; ++w) t += v[w];
+  return t;
+}
+
 // What bounds it: the read of both value arrays (134 M pairs: 168 us, 6.4 TB/s).
 // counts: [2][grid] kept pairs per CTA; totals: zeroed by the caller.
 __global__ void __launch_bounds__(kCompactThreads) compact_count_kernel(const float *__restrict__ vp,
@@ -90,55 +105,63 @@ __global__ void __launch_bounds__(kCompactThreads) compact_count_kernel(const fl
                                                                           long long *__restrict__ counts,
                                                                           unsigned *__restrict__ words,
                                                                           unsigned long long *__restrict__ totals) {
-  __shared__ unsigned long long s_cnt[2];
-  const int lane = threadIdx.x & 31;
-  if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0;
-  __syncthreads();
+  __shared__ long long s_cnt[2][kCompactWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const CompactRange r = compact_range(nb);
   long long mine = 0;
   for (long long b = r.b0; b < r.b1; ++b) {
-    const long long q = b * kCompactWarps + (threadIdx.x >> 5);
+    const long long q = b * kCompactWarps + warp;
     const unsigned word = compact_word(vp, vn, n, thr, q, lane);
     if (words) words[q * 32 + lane] = word;
     mine += __popc(word);
   }
-  if (mine) atomicAdd(&s_cnt[lane / kCompactWords], (unsigned long long)mine);
+  for (int o = kCompactWords / 2; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+  if (lane % kCompactWords == 0) s_cnt[lane / kCompactWords][warp] = mine;
   __syncthreads();
   if (threadIdx.x < 2) {
-    counts[(long long)threadIdx.x * gridDim.x + blockIdx.x] = (long long)s_cnt[threadIdx.x];
-    if (s_cnt[threadIdx.x]) atomicAdd(&totals[threadIdx.x], s_cnt[threadIdx.x]);
+    const long long all = warps_sum(s_cnt[threadIdx.x]);
+    counts[(long long)threadIdx.x * gridDim.x + blockIdx.x] = all;
+    if (all) atomicAdd(&totals[threadIdx.x], (unsigned long long)all);
   }
 }
 
 // The kept pairs of each chunk, one a lane: lane s takes the chunk's s-th kept
 // pair (a search over the words' running counts, then the bit of its rank), so
 // up to 32 gathers are in flight a warp and the stores are contiguous however
-// many are kept.  134 M pairs, 2 % kept: 238 us against 1514 with two
-// barriers per 256 pairs and 428 with a word at a time.  Without stored words
-// (a workspace that has no room for them) the values are read again.
-__global__ void __launch_bounds__(kCompactThreads) compact_write_kernel(
+// many are kept; a chunk with kCompactDense kept pairs or more goes word by word
+// instead.  134 M pairs, 2 % kept: 205 us (count and write 317) against 1514 with two
+// barriers per 256 pairs and 428 with a word at a time.  Small calls: a 64-bit shared atomicAdd a
+// thread for the counts of the CTAs before this one cost more than the gathers
+// (1 M pairs, count and write, 2 % kept 38.5 us, all kept 61; now 18 and 27).  WORDS: the stored
+// words are read, by 8 CTAs an SM (the whole grid resident; two rounds at a time and
+// 5 CTAs: 339 us).  Without them (a workspace that has no room) the values are
+// read again, 32 loads in flight a thread, which takes the registers of 5 CTAs.
+template <bool WORDS>
+__global__ void __launch_bounds__(kCompactThreads, WORDS ? 8 : 5) compact_write_kernel(
     const float *__restrict__ vp, const int *__restrict__ lp, const float *__restrict__ vn,
     const int *__restrict__ ln, long long n, float thr, long long nb, const long long *__restrict__ counts,
     const unsigned *__restrict__ words, long long capacity, long long *__restrict__ idx_p,
     float *__restrict__ val_p, int *__restrict__ lag_p, long long *__restrict__ idx_n, float *__restrict__ val_n,
     int *__restrict__ lag_n) {
-  __shared__ unsigned long long s_before[2];      // kept pairs of the CTAs before this one
-  __shared__ int s_warp[2][2][kCompactWarps];     // [block parity][side]: of each warp's chunk
+  __shared__ long long s_before[2][kCompactWarps];  // kept pairs of the CTAs before this one, by warp
+  __shared__ int s_warp[2][2][kCompactWarps];       // [block parity][side]: of each warp's chunk
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x < 2) s_before[threadIdx.x] = 0;
-  __syncthreads();
+  long long before[2] = {0, 0};
+  for (int c = threadIdx.x; c < (int)blockIdx.x; c += kCompactThreads) {
+    before[0] += counts[c];
+    before[1] += counts[(long long)gridDim.x + c];
+  }
+#pragma unroll
   for (int sd = 0; sd < 2; ++sd) {
-    unsigned long long t = 0;
-    for (int c = threadIdx.x; c < (int)blockIdx.x; c += kCompactThreads)
-      t += (unsigned long long)counts[(long long)sd * gridDim.x + c];
-    if (t) atomicAdd(&s_before[sd], t);
+    for (int o = 16; o > 0; o >>= 1) before[sd] += __shfl_xor_sync(0xffffffffu, before[sd], o);
+    if (lane == 0) s_before[sd][warp] = before[sd];
   }
   __syncthreads();
-  long long off_p = (long long)s_before[0], off_n = (long long)s_before[1];
+  long long off_p = warps_sum(s_before[0]), off_n = warps_sum(s_before[1]);
   const CompactRange r = compact_range(nb);
   for (long long b = r.b0; b < r.b1; ++b) {
     const long long q = b * kCompactWarps + warp;
-    const unsigned word = words ? __ldg(words + q * 32 + lane) : compact_word(vp, vn, n, thr, q, lane);
+    const unsigned word = WORDS ? __ldg(words + q * 32 + lane) : compact_word(vp, vn, n, thr, q, lane);
     const int c = __popc(word);
     int incl = c;  // running count over the 16 positive words, then the 16 negative ones
 #pragma unroll
@@ -162,38 +185,73 @@ __global__ void __launch_bounds__(kCompactThreads) compact_write_kernel(
         at_n += cnt[1][w];
       }
     }
-    for (int s0 = 0; s0 < all; s0 += 32) {
-      const int s = s0 + lane;
-      int k = 0;  // the word of the s-th kept pair: words whose running count is <= s
+    // rounds of up to 32 kept pairs, U at a time: their gathers are issued before the first store
+    auto rounds = [&](auto by_word, int n_rounds) {
+      constexpr int U = WORDS ? 1 : 2;
+      for (int r0 = 0; r0 < n_rounds; r0 += U) {
+        int at[U], rank[U];  // the pair within the chunk (word and bit; -1: none), and its rank among the kept
+        float val[U];
+        int lag[U];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const int x = __shfl_sync(0xffffffffu, incl, k + o - 1);
-        if (x <= s) k += o;
-      }
-      k = k < 31 ? k : 31;
-      const unsigned bits = __shfl_sync(0xffffffffu, word, k);
-      int rank = s - (__shfl_sync(0xffffffffu, incl, k) - __popc(bits));
-      if (s < all) {
-        int bit = 0;  // the set bit of that rank
+        for (int u = 0; u < U; ++u) {
+          at[u] = -1;
+          if (U > 1 && r0 + u >= n_rounds) continue;  // uniform
+          int k, bit, s;
+          bool kept;
+          if constexpr (by_word.value) {
+            k = r0 + u;
+            bit = lane;
+            const unsigned bits = __shfl_sync(0xffffffffu, word, k);
+            s = __shfl_sync(0xffffffffu, incl, k) - __popc(bits) + __popc(bits & ((1u << lane) - 1u));
+            kept = (bits >> lane) & 1u;
+          } else {
+            s = 32 * (r0 + u) + lane;
+            kept = s < all;
+            k = 0;  // the word of the s-th kept pair: words whose running count is <= s
 #pragma unroll
-        for (int w = 16; w > 0; w >>= 1) {
-          const int x = __popc((bits >> bit) & ((1u << w) - 1u));
-          if (rank >= x) {
-            rank -= x;
-            bit += w;
+            for (int w = 16; w > 0; w >>= 1) {
+              const int x = __shfl_sync(0xffffffffu, incl, k + w - 1);
+              if (x <= s) k += w;
+            }
+            k = k < 31 ? k : 31;
+            const unsigned bits = __shfl_sync(0xffffffffu, word, k);
+            int left = s - (__shfl_sync(0xffffffffu, incl, k) - __popc(bits));
+            bit = 0;  // the set bit of that rank
+#pragma unroll
+            for (int w = 16; w > 0; w >>= 1) {
+              const int x = __popc((bits >> bit) & ((1u << w) - 1u));
+              if (left >= x) {
+                left -= x;
+                bit += w;
+              }
+            }
+          }
+          const bool neg = s >= pos;
+          const int c = (k & (kCompactWords - 1)) * 32 + bit;
+          const long long e = q * (kCompactWords * 32) + c, o = neg ? at_n + (s - pos) : at_p + s;
+          // (e and o lie in range whenever the counts and words are those of these arrays)
+          if (kept && e < n && o >= 0 && o < capacity) {
+            at[u] = c;
+            rank[u] = s;
+            val[u] = __ldg((neg ? vn : vp) + e);
+            lag[u] = __ldg((neg ? ln : lp) + e);
           }
         }
-        const long long e = (q * kCompactWords + (k & (kCompactWords - 1))) * 32 + bit;
-        const bool neg = s >= pos;
-        const long long o = neg ? at_n + (s - pos) : at_p + s;
-        // (e and o lie in range whenever the counts and words are those of these arrays)
-        if (e < n && o >= 0 && o < capacity) {
-          (neg ? idx_n : idx_p)[o] = e;
-          (neg ? val_n : val_p)[o] = __ldg((neg ? vn : vp) + e);
-          (neg ? lag_n : lag_p)[o] = __ldg((neg ? ln : lp) + e);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (at[u] >= 0) {
+            const bool neg = rank[u] >= pos;
+            const long long o = neg ? at_n + (rank[u] - pos) : at_p + rank[u];
+            (neg ? idx_n : idx_p)[o] = q * (kCompactWords * 32) + at[u];
+            (neg ? val_n : val_p)[o] = val[u];
+            (neg ? lag_n : lag_p)[o] = lag[u];
+          }
         }
       }
-    }
+    };
+    if (all == 0) continue;  // uniform over the warp
+    if (all >= kCompactDense) rounds(std::true_type{}, 32);
+    else rounds(std::false_type{}, (all + 31) / 32);
   }
 }
 
@@ -309,10 +367,10 @@ static int compact_run(const float *d_vals_pos, const int *d_lags_pos, const flo
     note_launches(1);
   }
   if (e == cudaSuccess && capacity > 0) {
-    compact_write_kernel<<<grid, kCompactThreads, 0, st>>>(d_vals_pos, d_lags_pos, d_vals_neg, d_lags_neg, n_pairs,
-                                                           threshold, nb, counts, words, capacity, d_index_pos,
-                                                           d_value_pos, d_lag_pos, d_index_neg, d_value_neg,
-                                                           d_lag_neg);
+    const auto write = words ? compact_write_kernel<true> : compact_write_kernel<false>;
+    write<<<grid, kCompactThreads, 0, st>>>(d_vals_pos, d_lags_pos, d_vals_neg, d_lags_neg, n_pairs, threshold, nb,
+                                            counts, words, capacity, d_index_pos, d_value_pos, d_lag_pos,
+                                            d_index_neg, d_value_neg, d_lag_neg);
     e = cudaGetLastError();
     note_launches(1);
   }
