@@ -54,6 +54,7 @@
 #include "../../include/seismic_gb300.h"
 #include "energy.cuh"
 #include "kernels.cuh"
+#include "lag_items.cuh"
 #include "tcgen05.cuh"
 #include "tma_host.cuh"
 
@@ -936,32 +937,6 @@ static cudaError_t launch_lag_kernel(LagArgs &a, const LagPlan &pl, const unsign
   return cudaGetLastError();
 }
 
-// j's per work item: of 32, 16, ... 1 (multiples of jp, at most `most`), the
-// largest whose busiest CTA has the least to walk: its items' j's, and a
-// twentieth of a j an item with one plane (measured: N=6000, items of 1 for items of
-// 32 cost 2.3 % where they save 2.1 % of the j's; with two planes they cost nothing).
-// The strips and the A ring run on across items.  items(jc) counts the launch's
-// items.  5 queries against 6,177 x 3 events (lags +-256) ran as 49 items of 8 on 49 of
-// 150 SMs: 198 us, 147 items of 2: 91 us.  Triangle, three products, N=4001: 12.5 ->
-// 11.9 ms; N=600 556 -> 256 us.
-template <class F>
-static int lag_item_js(int most, int jp, int nhl, long long j_rows, int sm_count, F items) {
-  int best = jp;
-  long long best_cost = -1;
-  for (int jc = 32; jc >= jp; jc >>= 1) {
-    if (jc > most || jc % jp != 0) continue;
-    const long long n = items(jc);
-    const long long grid = n < sm_count ? n : sm_count;
-    if (grid <= 0) return jc;
-    const long long cost = (n + grid - 1) / grid * (20 * (jc < j_rows ? jc : j_rows) + (nhl == 1 ? 1 : 0));
-    if (best_cost < 0 || cost < best_cost) {
-      best = jc;
-      best_cost = cost;
-    }
-  }
-  return best;
-}
-
 long long lag_blocks(long long n) { return (n + kLagM - 1) / kLagM; }
 
 long long lag_block_row(long long b, long long n) { return b * kLagM < n ? b * kLagM : n; }
@@ -987,12 +962,8 @@ cudaError_t launch_lag_blocks(const void *ws, long long n, int C, int length, in
   a.L = length;
   a.shift = shift;
   a.nhl = nhl;
-  auto items_of = [&](int jc) {
-    long long items = 0;
-    for (long long bb = blk_begin; bb < blk_end; ++bb) items += (n - bb * kLagM + jc - 1) / jc;
-    return items;
-  };
-  a.jc = lag_item_js(pl.jc, pl.jp, nhl, n, sm_count, items_of);
+  auto items_of = [&](int jc) { return lag_triangle_items(n, kLagM, blk_begin, blk_end, jc); };
+  a.jc = lag_item_js(pl.jc, pl.jp, nhl, n, (long long)C * pl.lp * pl.wpad, sm_count, items_of);
   a.threshold = threshold;
   a.n_hist = n_hist;
   a.vals_pos = vp;
@@ -1033,7 +1004,7 @@ cudaError_t launch_lag_rect(const void *cat_ws, long long n_cat, const void *q_w
   const long long nblk = (n_cols + kLagM - 1) / kLagM;
   auto items_of = [&](int jc) { return nblk * ((n_query + jc - 1) / jc); };
   // at most 8 queries per item (4 and 8 measured equal for a 64-query request, 16 slower)
-  pl.jc = lag_item_js(8, pl.jp, nhl, n_query, sm_count, items_of);
+  pl.jc = lag_item_js(8, pl.jp, nhl, n_query, (long long)C * pl.lp * pl.wpad, sm_count, items_of);
   if (const char *env = getenv("SEISMIC_LAG_RECT_JC")) {  // 1 .. 64, a multiple of jp
     const int v = atoi(env);
     if (v >= 1 && v <= 64 && v % pl.jp == 0) pl.jc = v;
