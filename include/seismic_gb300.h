@@ -311,9 +311,13 @@ int seismic_tuning(int padded_size, int n_channels, int *tile, int *ctas_per_sm,
 /* The TMA-staged form's CTA shape the autotuner cached for exactly
  * (padded_size, n_channels spectrum rows per event): FFT warps per CTA (12,
  * or 99 for the widest CTA that keeps 128 registers a thread) and spectral
- * chunks per ring slot; both 0 when nothing is cached (the built-in rule
- * applies).  No counterpart in the reference. */
+ * chunks per ring slot (2, or 4 for 4 or more); both 0 when nothing is cached
+ * by this version of the kernel (the built-in rule applies).  No counterpart
+ * in the reference. */
 int seismic_tuning_staged(int padded_size, int n_channels, int *staged_warps, int *chunks_per_slot);
+/* The cached spectral chunks per ring slot themselves: 2, 4 or 8 (a whole
+ * spectrum row), 0 when nothing is cached. */
+int seismic_tuning_staged_slot(int padded_size, int n_channels, int *chunks);
 
 /* ---- serving loop --------------------------------------------------------
  * A catalog kept resident on the device as packed half spectra (FP32 or

@@ -45,6 +45,8 @@ def _declare(lib):
     lib.seismic_tuning_staged.restype = ctypes.c_int
     lib.seismic_tuning_staged.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_int),
                                           ctypes.POINTER(ctypes.c_int)]
+    lib.seismic_tuning_staged_slot.restype = ctypes.c_int
+    lib.seismic_tuning_staged_slot.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_int)]
     lib._batch_declared = True
     return lib
 
@@ -124,5 +126,7 @@ def tuning(padded_size: int, n_channels: int) -> dict:
     _lib.check(lib.seismic_tuning(padded_size, n_channels, ctypes.byref(t), ctypes.byref(c), ctypes.byref(i)))
     w, r = ctypes.c_int(), ctypes.c_int()
     _lib.check(lib.seismic_tuning_staged(padded_size, n_channels, ctypes.byref(w), ctypes.byref(r)))
+    s = ctypes.c_int()
+    _lib.check(lib.seismic_tuning_staged_slot(padded_size, n_channels, ctypes.byref(s)))
     return {"tile": t.value, "ctas_per_sm": c.value, "item_groups": i.value, "staged_warps": w.value,
-            "staged_ru": r.value}
+            "staged_ru": r.value, "staged_slot": s.value}

@@ -7,12 +7,16 @@
 //    couples share one event's spectrum in L1) and CTAs per SM;
 //  * the TMA-staged form (P = 512 .. 4096) over its CTA shapes: FFT warps
 //    per CTA (12, or the widest that keeps 128 registers a thread), which
-//    sets the pairs per work item, and spectral chunks per ring slot;
+//    sets the pairs per work item, and spectral chunks per ring slot (2, 4,
+//    and 8 where launches of this shape take them);
 //  * the batched kernel over work-item sizes (couples per item, in units of
 //    the CTA's groups).
 // The fastest parameters go into an in-process table (used by every later
 // launch in this process) and into a text cache file, one line per (P, C):
-//   P=<P> C=<C> tile=<t> ctas=<k> item=<g> us=<time> gpu=<name> warps=<w> ru=<r>
+//   P=<P> C=<C> tile=<t> ctas=<k> item=<g> us=<time> gpu=<name> warps=<w> ru=<r> slot=<s> rev=<v>
+// slot: the chunks per ring slot, ru: the same up to 4 (its former range), rev:
+// kStagedRevision.  The staged shape of a line of another revision, which was
+// timed on another kernel, is not used; its other parameters are.
 // Lookups of the direct-form and batched parameters fall back to (P, any C),
 // then to built-in defaults; the staged shape is used for the exact (P, C)
 // only.
@@ -32,6 +36,10 @@
 
 namespace seismic {
 namespace {
+
+// Raised when a change of the staged kernel moves what its CTA shapes are worth
+// (2: slots of a whole spectrum row, half-size exchanges, one arrive a warp).
+constexpr int kStagedRevision = 2;
 
 struct Entry {
   int P, C;
@@ -63,9 +71,12 @@ void load_file(const std::string &path) {
                &e.t.ctas_per_sm, &e.t.item_groups, &e.us, gpu) >= 5) {
       if (e.t.tile < 2 || e.t.tile > 64 || (e.t.tile & 1) || e.t.item_groups < 1) continue;
       const char *w = strstr(line, " warps=");
-      const char *r = strstr(line, " ru=");
-      e.t.staged_warps = w ? atoi(w + 7) : 0;
-      e.t.staged_ru = r ? atoi(r + 4) : 0;
+      const char *s = strstr(line, " slot=");
+      const char *v = strstr(line, " rev=");
+      const bool current = w && s && v && atoi(v + 5) == kStagedRevision;
+      e.t.staged_warps = current ? atoi(w + 7) : 0;
+      e.t.staged_ru = current ? atoi(s + 6) : 0;
+      if (e.t.staged_ru != 2 && e.t.staged_ru != 4 && e.t.staged_ru != 8) e.t.staged_ru = 0;
       e.gpu = gpu;
       bool replaced = false;
       for (auto &x : g_table)
@@ -96,9 +107,9 @@ bool write_file(const std::string &path) {
   FILE *f = fopen(path.c_str(), "w");
   if (!f) return false;
   for (const auto &e : g_table)
-    fprintf(f, "P=%d C=%d tile=%d ctas=%d item=%d us=%.1f gpu=%s warps=%d ru=%d\n", e.P, e.C, e.t.tile,
-            e.t.ctas_per_sm, e.t.item_groups, e.us, e.gpu.empty() ? "unknown" : e.gpu.c_str(), e.t.staged_warps,
-            e.t.staged_ru);
+    fprintf(f, "P=%d C=%d tile=%d ctas=%d item=%d us=%.1f gpu=%s warps=%d ru=%d slot=%d rev=%d\n", e.P, e.C,
+            e.t.tile, e.t.ctas_per_sm, e.t.item_groups, e.us, e.gpu.empty() ? "unknown" : e.gpu.c_str(),
+            e.t.staged_warps, std::min(e.t.staged_ru, 4), e.t.staged_ru, kStagedRevision);
   fclose(f);
   return true;
 }
@@ -167,7 +178,17 @@ extern "C" int seismic_tuning_staged(int padded_size, int n_channels, int *stage
   int w = 0, ru = 0;
   if (!tune_staged_lookup(padded_size, n_channels, &w, &ru)) w = ru = 0;
   if (staged_warps) *staged_warps = w;
-  if (chunks_per_slot) *chunks_per_slot = ru;
+  if (chunks_per_slot) *chunks_per_slot = std::min(ru, 4);
+  return SEISMIC_OK;
+}
+
+extern "C" int seismic_tuning_staged_slot(int padded_size, int n_channels, int *chunks) {
+  report_status(SEISMIC_OK, "");
+  if (!supported_padded_size(padded_size) || n_channels < 1)
+    return report_status(SEISMIC_ERR_UNSUPPORTED_SIZE, "unsupported padded size or channel count");
+  int w = 0, ru = 0;
+  if (!tune_staged_lookup(padded_size, n_channels, &w, &ru)) ru = 0;
+  if (chunks) *chunks = ru;
   return SEISMIC_OK;
 }
 
@@ -294,7 +315,8 @@ extern "C" int seismic_autotune(int padded_size, int n_channels, const char *cac
 
   // the staged form's CTA shape (FFT warps per CTA x chunks per ring slot)
   if (P >= 512 && P <= 4096 && staged_enabled()) {
-    const int shapes[4][2] = {{12, 4}, {12, 2}, {99, 4}, {99, 2}};  // 99: the widest CTA of this P
+    // 99: the widest CTA of this P
+    const int shapes[5][2] = {{12, 4}, {12, 2}, {99, 8}, {99, 4}, {99, 2}};
     double best_staged = 1e30;
     for (const auto &sh : shapes) {
       PairArgs sa2 = pa;
@@ -302,6 +324,7 @@ extern "C" int seismic_autotune(int padded_size, int n_channels, const char *cac
       sa2.staged_ru = sh[1];
       sa2.tile = bestT.tile;
       sa2.error_flag = err_flag;
+      if (staged_slot_chunks(P, sa2) != sh[1]) continue;  // such slots do not fit: timed as the shorter ones
       sa2.couple_begin = 0;
       sa2.couple_end = pair_work_total(P, sa2);
       double best = 1e30;

@@ -146,7 +146,8 @@ struct PairArgs {
   const void *spectra_i;
   int spec_channels;
   // Staged form: a CTA shape forced by the autotuner while it times the
-  // candidates (FFT warps per CTA, chunks per ring slot; 0 = not forced).
+  // candidates (FFT warps per CTA, chunks per ring slot: 2, 4 or 8; 0 = not
+  // forced).
   int staged_warps;
   int staged_ru;
   // Staged form, set by its launch: i and j events per work item (TI, TJ;
@@ -231,6 +232,8 @@ bool staged_enabled();
 long long staged_items_total(int P, const PairArgs &a);  // triangle or rectangle
 // Triangle walk of the staged form: events per tile side and work items per tile.
 void staged_tiling(int P, const PairArgs &a, long long *tile_side, long long *items_per_tile);
+// Chunks per ring slot (2, 4 or 8) of the launch that `a` makes.
+int staged_slot_chunks(int P, const PairArgs &a);
 // Launches items [a.couple_begin, a.couple_end) of the staged decomposition.
 cudaError_t launch_pairs_staged(int P, const PairArgs &a, int sm_count, cudaStream_t s);
 
@@ -290,7 +293,7 @@ struct TuneEntry {
   int ctas_per_sm;   // 0 = occupancy maximum
   int item_groups;   // couples per batched work item, in units of groups per CTA
   int staged_warps;  // staged form: FFT warps per CTA (0: the built-in rule)
-  int staged_ru;     // staged form, FP32 spectra: chunks per ring slot (0: the built-in rule)
+  int staged_ru;     // staged form, FP32 spectra: chunks per ring slot, 2, 4 or 8 (0: the built-in rule)
 };
 TuneEntry tune_lookup(int P, int n_channels);
 // The staged form's tuned CTA shape for exactly (P, spectrum rows), if any.

@@ -40,6 +40,15 @@ long long staged_items_total(int P, const PairArgs &a) {
 }
 
 cudaError_t launch_pairs_staged_large(int P, const PairArgs &a, int sm_count, cudaStream_t s);
+int staged_slot_chunks_large(int P, const PairArgs &a);
+
+int staged_slot_chunks(int P, const PairArgs &a) {
+  switch (P) {
+    case 512: return staged_choice<512>(a).ru;
+    case 1024: return staged_choice<1024>(a).ru;
+    default: return staged_slot_chunks_large(P, a);
+  }
+}
 
 cudaError_t launch_pairs_staged(int P, const PairArgs &a, int sm_count, cudaStream_t s) {
   switch (P) {

@@ -408,25 +408,24 @@ constexpr int kStagedWarps = 12;  // FFT warps per CTA, plus the producer warp
 // in whole groups of P/32 threads.
 constexpr int staged_wide_warps(int P) { return P >= 4096 ? 12 : (P == 2048 ? 14 : 15); }
 
-// CTA shape of a launch: FFT warps per CTA and chunks per ring slot.  In
-// order: a shape the autotuner forces while timing, SEISMIC_STAGED_WARPS
-// ("12", "wide") / SEISMIC_STAGED_RU ("2", "4", "8"), the tuner's cached choice
-// for exactly (P, spectrum rows), else the built-in rule: the wide CTA (the
-// most FFT warps that keep 128 registers a thread) with the longest slots that
-// launch_staged_p's rule takes (8 or 4 chunks).
+// CTA shape asked for a launch: FFT warps per CTA and chunks per ring slot (8:
+// the longest that fit, staged_choice).  In order: a shape the autotuner forces
+// while timing, SEISMIC_STAGED_WARPS ("12", "wide") / SEISMIC_STAGED_RU ("2",
+// "4", "8"), the tuner's cached choice for exactly (P, spectrum rows; its
+// chunks, timed on FP32 spectra, for those alone), else the built-in rule: the
+// wide CTA (the most FFT warps that keep 128 registers a thread) with the
+// longest slots.
 // Measured with items of TI x TJ events, FP32, ms, 12 warps / wide:
 // overlap-save Q=512 x 4 rows (N=6000) 20.2 / 17.5, Q=1024 x 2 frames of three
 // channels (N=3000) 12.3 / 10.0, P=512 (N=3000) 3.50 / 3.23, P=1024 6.25 / 5.86, P=2048 with
 // three channels (N=2000) 8.25 / 7.44 (P=4096: the same
-// CTA).  Half-precision spectra take no 2-chunk slots; an FP32 launch
-// whose item rows leave no room for two 4-chunk slots takes 2
-// (launch_staged_p).
+// CTA).  Half-precision spectra take no 2-chunk slots.
 struct StagedShape {
   int nwarp, ru;
 };
 static StagedShape staged_shape(int P, const PairArgs &a) {
   const int rows = spectrum_rows(a);
-  int w = a.staged_warps, ru = a.staged_ru == 4 ? 8 : a.staged_ru;  // the tuner times 2 chunks against the rule's
+  int w = a.staged_warps, ru = a.staged_ru;
   if (!w) {
     const char *e = getenv("SEISMIC_STAGED_WARPS");
     if (e && strcmp(e, "wide") == 0) w = staged_wide_warps(P);
@@ -441,7 +440,7 @@ static StagedShape staged_shape(int P, const PairArgs &a) {
   int tw = 0, tru = 0;
   if ((!w || !ru) && tune_staged_lookup(P, rows, &tw, &tru)) {
     if (!w) w = tw;
-    if (!ru) ru = tru == 2 ? 2 : 0;
+    if (!ru && a.stype == 0) ru = tru;
   }
   if (!w) w = staged_wide_warps(P);
   w = (w == kStagedWarps) ? kStagedWarps : staged_wide_warps(P);
@@ -558,48 +557,72 @@ constexpr int default_item_rows(int ng) {
   return best;
 }
 
-template <int P> static cudaError_t launch_staged_p(const PairArgs &a, int sm_count, cudaStream_t s) {
+// Ring slots of `ru` chunks that a launch has room for (0: no such form).
+template <int P> static int staged_slots(const PairArgs &a, bool wide, int ru) {
+  constexpr int WW = staged_wide_warps(P);
+  if (ru == 8) {
+    if constexpr (P <= 2048)
+      if (wide)
+        return a.stype == 0 ? staged_ring_slots<P, WW, 8, 0>(a, nullptr) : staged_ring_slots<P, WW, 8, 1>(a, nullptr);
+    return 0;
+  }
+  if (a.stype != 0)
+    return ru != 4 ? 0
+           : wide  ? staged_ring_slots<P, WW, 4, 1>(a, nullptr)
+                   : staged_ring_slots<P, kStagedWarps, 4, 1>(a, nullptr);
+  if (ru == 4)
+    return wide ? staged_ring_slots<P, WW, 4, 0>(a, nullptr) : staged_ring_slots<P, kStagedWarps, 4, 0>(a, nullptr);
+  return wide ? staged_ring_slots<P, WW, 2, 0>(a, nullptr) : staged_ring_slots<P, kStagedWarps, 2, 0>(a, nullptr);
+}
+
+// The form that a launch takes: the wide or the 12-warp CTA, whether its item
+// geometry is the compile-time one (the default CTA with its default items),
+// and the chunks per ring slot: those asked for, down to what fits.
+// 8 chunks, a whole spectrum row, are taken where the ring holds
+// three such slots, or two and an event has one row.  Every unit costs its
+// wait, vote and arrive: 2-chunk slots run 6-21 % slower than 4-chunk ones,
+// 8-chunk ones faster still (ms, 4 / 8 chunks): Q=512 x 4 17.46 / 16.35, FP16
+// 17.06 / 15.77, Q=1024 x 2 frames of three channels 10.03 / 9.81, P=1024 with three
+// channels 5.35 / 5.15, P=2048 12.61 / 11.90 (with three channels, two slots, 7.43 / 7.51: four).
+// FP32 spectra whose item rows leave no room for two 4-chunk slots take 2.
+struct StagedChoice {
+  bool wide, ct;
+  int ru;
+};
+template <int P> static StagedChoice staged_choice(const PairArgs &a) {
+  constexpr int WW = staged_wide_warps(P);
+  constexpr int NG = WW * 32 / (P / 32);
   const StagedShape sh = staged_shape(P, a);
+  StagedChoice c{sh.nwarp == WW, false, sh.ru};
+  c.ct = c.wide && staged_item_rows(NG, a) == default_item_rows(NG);
+  if (c.ru == 8) {
+    const int k = c.ct ? staged_slots<P>(a, c.wide, 8) : 0;
+    if (!(k >= 3 || (k == 2 && spectrum_rows(a) == 1))) c.ru = 4;
+  }
+  if (c.ru == 4 && a.stype == 0 && staged_slots<P>(a, c.wide, 4) < 2) c.ru = 2;
+  return c;
+}
+
+template <int P, int ST>
+static cudaError_t launch_staged_st(const PairArgs &a, const StagedChoice &c, int sm_count, cudaStream_t s) {
   constexpr int WW = staged_wide_warps(P);
   constexpr int KT = default_item_rows(WW * 32 / (P / 32));
-  const bool wide = sh.nwarp == WW;
-  // the default CTA with its default item geometry: the compile-time form
-  const bool ct = wide && staged_item_rows(WW * 32 / (P / 32), a) == KT;
-  // The default slot: all eight chunks of a spectrum row, where the ring holds
-  // three such slots, or two and an event has one row.  Every unit costs its
-  // wait, vote and arrive: 2-chunk slots run 6-21 % slower than 4-chunk ones,
-  // 8-chunk ones faster still (ms, 4 / 8 chunks): Q=512 x 4 17.46 / 16.35, FP16
-  // 17.06 / 15.77, Q=1024 x 2 frames of three channels 10.03 / 9.81, P=1024 with three
-  // channels 5.35 / 5.15, P=2048 12.61 / 11.90 (with three channels, two slots, 7.43 / 7.51: four).
-  if constexpr (P <= 2048) {
-    auto fits = [&](int k) { return k >= 3 || (k == 2 && spectrum_rows(a) == 1); };
-    if (ct && sh.ru == 8) {
-      if (a.stype == 0 && fits(staged_ring_slots<P, WW, 8, 0>(a, nullptr)))
-        return launch_staged_t<P, WW, 8, 0, KT>(a, sm_count, s);
-      if (a.stype == 1 && fits(staged_ring_slots<P, WW, 8, 1>(a, nullptr)))
-        return launch_staged_t<P, WW, 8, 1, KT>(a, sm_count, s);
-      if (a.stype == 2 && fits(staged_ring_slots<P, WW, 8, 2>(a, nullptr)))
-        return launch_staged_t<P, WW, 8, 2, KT>(a, sm_count, s);
-    }
-  }
+  if constexpr (P <= 2048)
+    if (c.ru == 8) return launch_staged_t<P, WW, 8, ST, KT>(a, sm_count, s);
+  if constexpr (ST == 0)
+    if (c.ru == 2)
+      return c.wide ? launch_staged_t<P, WW, 2, 0, 0>(a, sm_count, s)
+                    : launch_staged_t<P, kStagedWarps, 2, 0, 0>(a, sm_count, s);
+  if (!c.wide) return launch_staged_t<P, kStagedWarps, 4, ST, 0>(a, sm_count, s);
+  return c.ct ? launch_staged_t<P, WW, 4, ST, KT>(a, sm_count, s) : launch_staged_t<P, WW, 4, ST, 0>(a, sm_count, s);
+}
+
+template <int P> static cudaError_t launch_staged_p(const PairArgs &a, int sm_count, cudaStream_t s) {
+  const StagedChoice c = staged_choice<P>(a);
   switch (a.stype) {
-    case 0:
-      if (wide) {
-        if (sh.ru != 2 && staged_ring_slots<P, WW, 4, 0>(a, nullptr) >= 2)
-          return ct ? launch_staged_t<P, WW, 4, 0, KT>(a, sm_count, s) : launch_staged_t<P, WW, 4, 0, 0>(a, sm_count, s);
-        return launch_staged_t<P, WW, 2, 0, 0>(a, sm_count, s);
-      }
-      return (sh.ru != 2 && staged_ring_slots<P, kStagedWarps, 4, 0>(a, nullptr) >= 2)
-                 ? launch_staged_t<P, kStagedWarps, 4, 0, 0>(a, sm_count, s)
-                 : launch_staged_t<P, kStagedWarps, 2, 0, 0>(a, sm_count, s);
-    case 1:
-      if (wide)
-        return ct ? launch_staged_t<P, WW, 4, 1, KT>(a, sm_count, s) : launch_staged_t<P, WW, 4, 1, 0>(a, sm_count, s);
-      return launch_staged_t<P, kStagedWarps, 4, 1, 0>(a, sm_count, s);
-    case 2:
-      if (wide)
-        return ct ? launch_staged_t<P, WW, 4, 2, KT>(a, sm_count, s) : launch_staged_t<P, WW, 4, 2, 0>(a, sm_count, s);
-      return launch_staged_t<P, kStagedWarps, 4, 2, 0>(a, sm_count, s);
+    case 0: return launch_staged_st<P, 0>(a, c, sm_count, s);
+    case 1: return launch_staged_st<P, 1>(a, c, sm_count, s);
+    case 2: return launch_staged_st<P, 2>(a, c, sm_count, s);
     default: return cudaErrorInvalidValue;
   }
 }
