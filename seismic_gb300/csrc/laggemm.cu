@@ -53,6 +53,7 @@
 
 #include "../../include/seismic_gb300.h"
 #include "energy.cuh"
+#include "hist_bin.cuh"
 #include "kernels.cuh"
 #include "lag_items.cuh"
 #include "tcgen05.cuh"
@@ -223,12 +224,6 @@ __device__ __forceinline__ bool builders_all(bool ok) {
       : "r"((uint32_t)ok)
       : "memory");
   return r != 0;
-}
-
-__device__ __forceinline__ int hist_bin_lag(float v, float delta, int n_hist) {
-  if (v >= 1.0f) return n_hist - 1;
-  int b = (int)(v / delta);
-  return b > n_hist - 1 ? n_hist - 1 : (b < 0 ? 0 : b);
 }
 
 // Column n of a pass is lag shift - n (triangle: n increasing = lag
@@ -744,8 +739,8 @@ __global__ void __launch_bounds__(kLagThreads, 1)
               lp = best > 0.f ? lag0 + dir * bn : 0;
               ln = worst < 0.f ? lag0 + dir * wn : 0;
               if (a.n_hist > 0) {
-                const int hp = hist_bin_lag(vp, a.delta_hist, a.n_hist);
-                const int hn = hist_bin_lag(-vn, a.delta_hist, a.n_hist);
+                const int hp = hist_bin_div(vp, a.delta_hist, a.n_hist);
+                const int hn = hist_bin_div(-vn, a.delta_hist, a.n_hist);
                 if (smem_hist) {
                   atomicAdd(&hist[hp], 1);
                   atomicAdd(&hist[a.n_hist + hn], 1);

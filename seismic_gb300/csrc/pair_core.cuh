@@ -28,6 +28,7 @@
 #include <climits>
 
 #include "fft_core.cuh"
+#include "hist_bin.cuh"
 #include "kernels.cuh"
 
 namespace seismic {
@@ -150,19 +151,6 @@ __device__ __forceinline__ float2 product_pair(float2 a, float2 b) {
 }
 // x (s.x + s.y) rounded once to float (up to a rare double rounding).
 __device__ __forceinline__ float compensated_scale(float x, float2 s) { return fmaf(x, s.x, x * s.y); }
-
-// Bin of a coefficient v >= 0: (int)(v / delta), the quotient rounded to
-// nearest as the division gives it, without its instructions (45 an IEEE
-// division, measured): with inv the correctly rounded 1 / delta, one
-// residual step on v inv is the correctly rounded quotient (Markstein's
-// theorem, P. Markstein, "Computation of elementary functions on the IBM
-// RISC System/6000", 1990).
-__device__ __forceinline__ int hist_bin(float v, float delta, float inv, int n_hist) {
-  if (v >= 1.0f) return n_hist - 1;
-  const float q = v * inv;
-  const int b = (int)fmaf(fmaf(-q, delta, v), inv, q);
-  return b > n_hist - 1 ? n_hist - 1 : (b < 0 ? 0 : b);
-}
 
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float r;

@@ -22,6 +22,7 @@
 #include <type_traits>
 
 #include "../../include/seismic_gb300.h"
+#include "hist_bin.cuh"
 #include "kernels.cuh"
 
 namespace seismic {
@@ -42,16 +43,6 @@ constexpr int kCompactBlock = kCompactWarps * kCompactWords * 32;     // pairs p
 constexpr int kHistThreads = 256;
 constexpr int kHistSmemMax = 4096;
 constexpr int kHistSmemBytes = 48 * 1024;
-
-// Bin of a stored coefficient, the pair kernel's rule: (int)(v / delta) with
-// the quotient rounded to nearest, by a correctly rounded reciprocal and one
-// residual step (Markstein's theorem; hist_bin in pair_core.cuh).
-__device__ __forceinline__ int sparse_hist_bin(float v, float delta, float inv, int n_hist) {
-  if (v >= 1.0f) return n_hist - 1;
-  const float q = v * inv;
-  const int b = (int)fmaf(fmaf(-q, delta, v), inv, q);
-  return b > n_hist - 1 ? n_hist - 1 : (b < 0 ? 0 : b);
-}
 
 // The blocks that this CTA owns, a contiguous run; warp w takes chunk (512
 // pairs) w of each, so a CTA reads 16 KB runs (a run of chunks per warp read 134
@@ -271,8 +262,8 @@ __global__ void __launch_bounds__(kHistThreads) histogram_kernel(const float *__
   __syncthreads();
   const int mine = rep ? (int)threadIdx.x & (rep - 1) : 0;
   auto count = [&](float p, float m) {
-    const int hp = sparse_hist_bin(p, delta, inv, n_hist);
-    const int hn = sparse_hist_bin(-m, delta, inv, n_hist);
+    const int hp = hist_bin(p, delta, inv, n_hist);
+    const int hn = hist_bin(-m, delta, inv, n_hist);
     if (rep) {
       atomicAdd(&s_hist[hp * rep + mine], 1);
       atomicAdd(&s_hist[(n_hist + hn) * rep + mine], 1);
