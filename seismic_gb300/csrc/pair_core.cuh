@@ -402,15 +402,20 @@ template <int P> __device__ __forceinline__ uint32_t window_mask(int t, int shif
 // 20.5 / 16.2.
 
 // Prescaled liveness by the copy-and-vote path of scan_and_write (VOTE), or
-// by thread 0's loads in the epilogue.  Measured, M pairs/s, vote vs loads:
-// FP32 spectra N=4096 C=3 P=4096 94.7 vs 91.5; FP16 there 93.4 vs 102.4; FP32
-// at N=16384 P=512 (not prescaled; the code alone) 825 vs 831.
+// by loads of the finishing threads in the epilogue.  The line was drawn when
+// one thread did those loads.  Measured with four, ms, vote / loads: FP32, three
+// channels, P=1024 (N=2000) 3.32 / 3.20, P=2048 (N=1500) 4.25 / 4.17, P=4096 (N=1200) 5.85 /
+// 5.88, Q=1024 x 2 frames (N=2500) 6.80 / 6.72; one channel, where only the code is in the
+// way, P=1024 (N=3000) 5.75 / 5.62, P=4096 (N=1500) 7.22 / 6.70; P=512 3.21 / 3.09.  FP16 with
+// three channels P=1024 3.16 / 3.06, P=4096 5.52 / 5.78.  So the vote is still the faster
+// side at P = 4096 with several channels alone.
 template <int P, int ST> constexpr bool kLivenessVote = ST == 0 && P >= 1024;
 
 // A thread's 32 last-pass values v[q RL + r] in four blocks of eight for the
 // scan: block b holds the rows r in [b RL/4, (b + 1) RL/4), every job q.
 // Rows lie P/RL lags apart, so a short window leaves whole blocks outside it
-// (at Q = 512 and +-128 lags, blocks 1 and 2).
+// (at Q = 512 and +-128 lags block 2; of block 1 it holds one value, lag +128, the
+// first of each group's thread 0).
 template <int RL> __host__ __device__ constexpr bool in_scan_block(int e, int b) { return (e % RL) / (RL / 4) == b; }
 template <int RL> __host__ __device__ constexpr uint32_t scan_block_bits(int b) {
   uint32_t m = 0;
@@ -422,7 +427,8 @@ template <int RL> __host__ __device__ constexpr uint32_t scan_block_bits(int b) 
 // STRAIGHT: the lag search straight through a thread's values (all owners of a
 // warp in step), else block by block.  The staged form searches straight: ms,
 // blocks / straight, P=1024 5.99 / 5.86, Q=1024 x 2 frames of three channels 10.39 /
-// 10.04, Q=512 x 4 17.61 / 17.47, P=4096 13.44 / 13.00, P=2048 12.56 / 12.63.  The direct
+// 10.04, Q=512 x 4 17.61 / 17.47, P=4096 13.44 / 13.00, P=2048 (N=2000) 5.69 / 5.35 (with three
+// channels 4.21 / 4.25).  The direct
 // form by blocks: P=256 2.04 / 2.07, P=8192 6.39 / 7.36 (three channels 8.7 / 12.4), the batch 34.2 / 35.3.
 template <int P, bool VOTE, bool STRAIGHT>
 __device__ __forceinline__ void scan_and_write(const PairArgs &a, float2 (&v)[32], long long ia, long long ja,
@@ -452,7 +458,7 @@ __device__ __forceinline__ void scan_and_write(const PairArgs &a, float2 (&v)[32
   // nonzero.  Lane c < VL of the group copies channel c's inverse norms of
   // i, ja, jb into the group's exchange buffer by cp.async (the buffer is
   // free after the transform's last barrier) and a vote after the scan
-  // combines them (channels from VL on: thread 0 below).  No loads on the
+  // combines them (channels from VL on: the finishing threads below).  No loads on the
   // epilogue's path and no registers held across the scan.
   constexpr int VL = G < 32 ? G : 32;
   float *chn = reinterpret_cast<float *>(xbuf);

@@ -16,12 +16,14 @@
 // catalog) walks column blocks of TJ events, all query blocks per column
 // block.
 //
-// Pipeline.  Each item's spectra are cut into units (channel c, chunk r):
-// bins [r S, (r+1) S) of the TI rows i0.. and the TJ rows j0.., exactly the
-// bins ca + r S and cb + r S every FFT thread reads at step r
-// (pair_core.cuh).  A producer warp (one elected thread) streams units into
-// a ring of K shared-memory slots: two 3-D TMA boxes {S bins, 1 channel, TI
-// or TJ events} (rows past the last event are zero-filled by the TMA unit),
+// Pipeline.  A spectrum row is eight chunks of S bins, chunk r holding exactly
+// the bins ca + r S and cb + r S that every FFT thread reads at step r
+// (pair_core.cuh).  Each item's spectra are cut into units (channel c, RU
+// consecutive chunks): their bins of the TI rows i0.. and the TJ rows j0...  A
+// producer warp (one elected thread) streams units into a ring of K
+// shared-memory slots by 3-D TMA boxes {BX chunks, 1 channel, TI or TJ events},
+// two (the i and the j rows) for every BX of the unit's chunks, BX S at most 256
+// bins (rows past the last event are zero-filled by the TMA unit),
 // completing on the slot's `full` mbarrier; the FFT warps conj-multiply
 // from the slot and release it on its `empty` mbarrier, one arrive a warp.  While the groups
 // run their inverse FFTs the producer fills the ring with the next item's
@@ -82,7 +84,9 @@ template <int P, int NWARP, int RU, int ST> struct Staged {  // RU: chunks r per
   // before / after: Q=1024 x 2 frames of three channels (N=3000) 12.4 / 10.4, plain P=2048
   // with three channels (N=2000) 8.86 / 7.39, P=2048 (N=3000) 13.6 / 12.6, Q=512 x 4
   // (N=6000) 18.5 / 17.6, P=1024 with three channels (N=2500) 5.69 / 5.46.  Half types' items
-  // are half as long and gain nothing from a deeper ring (FP16 Q=512 x 4 17.28 / 17.39).
+  // are half as long; full / split exchange, FP16: P=512 3.05 / 3.21, P=1024 5.58 / 5.73, P=2048 5.42 /
+  // 5.51, P=4096 7.10 / 7.24, Q=512 x 4 10.92 / 11.22, P=1024 with three channels 3.06 / 3.14.  Only with three
+  // channels at P=2048 (3.97 / 3.76) and P=4096 (5.78 / 5.53) would the deeper ring be the faster side.
   static constexpr bool SPLIT_EX = ST == 0;
   static constexpr int EX_LEN = SPLIT_EX ? padded_len<P / 2>() : padded_len<P>();
   static constexpr size_t EX_BYTES = (size_t)NG * EX_LEN * sizeof(float2);
